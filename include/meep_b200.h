@@ -551,6 +551,13 @@ int mtb_yee3d_set_slab(mtb_yee3d_plan *plan, int32_t own_lo, int32_t own_hi);
 int mtb_yee3d_begin(mtb_yee3d_plan *plan, int64_t t0, int32_t k, const double *coef,
                     void *stream);
 int mtb_yee3d_half(mtb_yee3d_plan *plan, int32_t part, void *stream);
+/* As mtb_yee3d_run for k steps on the split kernels, without plane samples, keeping E
+ * for the adjoint: E component c (0..2) before the first step at rec + c *
+ * rec_comp_stride and after step q (0-based) at rec + (q + 1) * rec_slot_stride + c *
+ * rec_comp_stride (box layout, 16-byte aligned). The steps write E there directly. */
+int mtb_yee3d_run_record(mtb_yee3d_plan *plan, int64_t t0, int32_t k, const double *coef,
+                         float *rec, int64_t rec_comp_stride, int64_t rec_slot_stride,
+                         void *stream);
 int32_t mtb_yee3d_current(const mtb_yee3d_plan *plan);
 int64_t mtb_yee3d_last_launches(const mtb_yee3d_plan *plan);
 int mtb_yee3d_set_timing(mtb_yee3d_plan *plan, int32_t enable);
@@ -589,6 +596,10 @@ int mtb_yee3d_adjoint_create(const mtb_yee3d_struct *s, const mtb_adj3d_buffers 
  * t0+q-1. */
 int mtb_yee3d_adjoint_run(mtb_yee3d_adjoint *p, int64_t t0, int32_t k, const float *rec,
                           int64_t rec_comp_stride, int64_t rec_slot_stride, void *stream);
+/* only_layers != 0: g_psi is kept inside the CPML layers only (where its profile has
+ * a != 0; elsewhere it feeds nothing back), which saves its traffic outside them.
+ * Default 0: g_psi is d J / d psi everywhere. */
+int mtb_yee3d_adjoint_psi_layers(mtb_yee3d_adjoint *p, int32_t only_layers);
 int64_t mtb_yee3d_adjoint_last_launches(const mtb_yee3d_adjoint *p);
 void mtb_yee3d_adjoint_destroy(mtb_yee3d_adjoint *p);
 

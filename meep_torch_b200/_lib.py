@@ -140,6 +140,8 @@ SIGNATURES = {
                                         C.POINTER(PhaseGroup), C.c_int32, C.c_int64,
                                         C.POINTER(Tuning), C.POINTER(vp)]),
     "mtb_yee3d_run": (C.c_int, [vp, C.c_int64, C.c_int32, C.POINTER(C.c_double), vp]),
+    "mtb_yee3d_run_record": (C.c_int, [vp, C.c_int64, C.c_int32, C.POINTER(C.c_double), vp,
+                                       C.c_int64, C.c_int64, vp]),
     "mtb_yee3d_check": (C.c_int, [vp, vp]),
     "mtb_yee3d_set_slab": (C.c_int, [vp, C.c_int32, C.c_int32]),
     "mtb_yee3d_begin": (C.c_int, [vp, C.c_int64, C.c_int32, C.POINTER(C.c_double), vp]),
@@ -152,6 +154,7 @@ SIGNATURES = {
                                            C.POINTER(PhaseGroup), C.c_int32, C.c_int64,
                                            C.c_int32, C.POINTER(vp)]),
     "mtb_yee3d_adjoint_run": (C.c_int, [vp, C.c_int64, C.c_int32, vp, C.c_int64, C.c_int64, vp]),
+    "mtb_yee3d_adjoint_psi_layers": (C.c_int, [vp, C.c_int32]),
     "mtb_yee3d_adjoint_last_launches": (C.c_int64, [vp]),
     "mtb_yee3d_adjoint_destroy": (None, [vp]),
     "mtb_yee3d_set_timing": (C.c_int, [vp, C.c_int32]),

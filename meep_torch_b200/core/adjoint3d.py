@@ -79,6 +79,8 @@ def run_3d_adjoint(c, n_steps: int, chunk: int, source, monitors, loss_fn, state
                                              regs if nreg else None, nreg, eng.groups,
                                              eng.n_groups, eng.ring_elems, K, C.byref(adj)),
                 "mtb_yee3d_adjoint_create")
+        # d J / d psi is not returned: it is only needed where it feeds back
+        L.check(lib.mtb_yee3d_adjoint_psi_layers(adj, 1), "mtb_yee3d_adjoint_psi_layers")
         keep = [gf, gpsi, tmp, geps, g_accs, gpol]
         N = nx * ny * zp
         record = torch.empty((K + 1, 3, nx, ny, zp), dtype=torch.float32, device=dev)
@@ -87,12 +89,7 @@ def run_3d_adjoint(c, n_steps: int, chunk: int, source, monitors, loss_fn, state
         for ci in range(len(chunks) - 1, -1, -1):
             s0, k = chunks[ci]
             rec.restore(snaps[ci])
-            for cc, t in enumerate(rec.live_e()):
-                record[0, cc].copy_(t)
-            for q in range(k):
-                rec.run(s0 + q, 1)
-                for cc, t in enumerate(rec.live_e()):
-                    record[q + 1, cc].copy_(t)
+            rec.run_record(s0, k, record)
             L.check(lib.mtb_yee3d_adjoint_run(adj, s0, k, L.ptr(record), N, 3 * N, stream),
                     "mtb_yee3d_adjoint_run")
         g_eps = eng._unpack(geps, (nx, ny, nz))

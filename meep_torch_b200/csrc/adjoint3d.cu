@@ -9,21 +9,26 @@
 // carries.
 //
 // Reverse of forward step t, adjoint state A = d J / d state_{t+1} on entry:
-//   k_adj3_inject  monitor plane samples of state_{t+1} -> gE, gH (scatter)
-//   k_adj3_e       E' = E + (dt curl + s) / eps_c:
-//                    d J / d eps_c = -gE' (E' - E) / eps_c       -> tmp6..8
-//                    g_curl = dt gE' / eps_c on the curl interior
-//                    E-side psi transposes -> g_psi6..11, adjoints of the six
-//                    H differences -> tmp0..5; gE passes through (identity)
-//   k_adj3_h       gH += transposed differences of tmp0..5; H' = H - dt curl E:
-//                    H-side psi transposes -> g_psi0..5, adjoints of the six E
-//                    differences -> tmp9..14
-//   k_adj3_fin     gE += transposed differences of tmp9..14;
-//                  g_eps += the two cells of each Yee average (tmp6..8)
+//   inject  monitor plane samples of state_{t+1} -> gE, gH (scatter)
+//   E part  E' = E + (dt curl + s) / eps_c:
+//             d J / d eps_c = -gE' (E' - E) / eps_c, its numerator summed over the
+//             steps of a run                               -> tmp6..8
+//             g_curl = dt gE' / eps_c on the curl interior
+//             E-side psi transposes -> g_psi6..11, adjoints of the six
+//             H differences -> tmp0..5; gE passes through (identity)
+//   H part  gH += transposed differences of tmp0..5; H' = H - dt curl E:
+//             H-side psi transposes -> g_psi0..5, adjoints of the six E
+//             differences -> tmp9..14
+//   fin     gE += transposed differences of tmp9..14
+// After the steps of a run, k_adj3_eps divides tmp6..8 by the averages and gathers the
+// two cells of each Yee average into g_eps: the average is linear, so one gather of the
+// sum replaces one per step.
 // tmp index: 0 Ex:dy(Hz) 1 Ex:dz(Hy) 2 Ey:dz(Hx) 3 Ey:dx(Hz) 4 Ez:dx(Hy)
 // 5 Ez:dy(Hx) 6 eps_x 7 eps_y 8 eps_z 9 Hx:dy(Ez) 10 Hx:dz(Ey) 11 Hy:dz(Ex)
-// 12 Hy:dx(Ez) 13 Hz:dx(Ey) 14 Hz:dy(Ex); a tmp array is zero outside the
-// cells where its term exists.
+// 12 Hy:dx(Ez) 13 Hz:dx(Ey) 14 Hz:dy(Ex); tmp0..5 and 9..14 are zero outside the
+// cells where their term exists.
+// Launches per step: H part, inject, and fin of the step with the E part of the one
+// before it (k_adj3_fe): both touch only their own node, so gE makes one round trip.
 #include <algorithm>
 #include <vector>
 
@@ -31,7 +36,7 @@
 
 namespace mtb {
 
-constexpr int A3Y = 8;            // y rows per block (warp = 128 z of one row)
+constexpr int A3_T = 128;         // float4s per block, three components each
 
 struct Adj3 {
     mtb_adj3d_buffers b;
@@ -43,6 +48,7 @@ struct Adj3 {
     float c1[MTB_MAX_POLES], c2[MTB_MAX_POLES];
     int np;                       // dispersive poles (0: none)
     int pmc;                      // PMC walls: bit 0 x, 1 y, 2 z
+    int psi_all;                  // 1: g_psi outside the layers too (adjoint_psi_layers)
     int nx, ny, nz, zp;
     float dt, rdx;
 };
@@ -84,296 +90,330 @@ __global__ void k_adj3_inject(const mtb_yee3d_struct *__restrict__ SS,
               radj[S.plane_ring_off[lo] + p]);
 }
 
-__global__ void __launch_bounds__(32 * A3Y) k_adj3_e(const __grid_constant__ Adj3 P,
-                                                    const float *__restrict__ en_,
-                                                    const float *__restrict__ eo_,
-                                                    int64_t rec_comp) {
+// The adjoint kernels take a float4 of z of one component per thread (threadIdx.y the
+// component, blockIdx.y the x plane, threadIdx.x counting float4s through the plane's
+// rows). All three components in one thread took 158 (E) and 128 (H) registers and one
+// or two blocks an SM, with the loads' latency exposed: E 52.3 us, H 12.4 us on
+// 96 x 80 x 72.
+struct A3Cell {
+    int i, j, kb, lane;
+    uint32_t g;
+    bool act;
+    __device__ __forceinline__ A3Cell(const Adj3 &P) {
+        const uint32_t zq = (uint32_t)P.zp >> 2;
+        const uint32_t q = blockIdx.x * (uint32_t)A3_T + threadIdx.x;
+        act = q < (uint32_t)P.ny * zq;
+        i = blockIdx.y;
+        j = (int)(q / zq);
+        kb = 4 * (int)(q - (uint32_t)j * zq);
+        lane = threadIdx.x & 31;
+        g = (uint32_t)i * ((uint32_t)P.ny * P.zp) + 4u * q;
+    }
+};
+
+// CPML profile (b, a) of one node, (1, 0) where it is not applied
+__device__ __forceinline__ void a3_prof(const Adj3 &P, int ax, int h, bool on, int k, float &b,
+                                        float &a) {
+    b = prof(P.pb[ax][h], on, 1.f, k);
+    a = prof(P.pa[ax][h], on, 0.f, k);
+}
+
+// gE of component C: += the transposed differences of the H part's adjoints (fin).
+template <int C>
+__device__ __forceinline__ void a3_fin(const Adj3 &P, const A3Cell &c, float (&ge)[4]) {
+    // Ex: dz(Ex) of Hy (11), dy(Ex) of Hz (14); Ey: dz(Ey) of Hx (10), dx(Ey) of Hz (13);
+    // Ez: dy(Ez) of Hx (9), dx(Ez) of Hy (12)
+    constexpr int UA = C == 0 ? 11 : C == 1 ? 10 : 9, UB = C == 0 ? 14 : C == 1 ? 13 : 12;
+    const int ZP = P.zp;
+    const uint32_t g = c.g, NYZ = (uint32_t)P.ny * ZP;
+    float ua[4], uap[4], ub[4], ubp[4], zk = 0.f;
+    zz(ua); zz(uap); zz(ub); zz(ubp);
+    if (c.act) {
+        l4(P.b.tmp[UA] + g, ua);
+        l4(P.b.tmp[UB] + g, ub);
+        if (C == 2 && c.j >= 1) l4(P.b.tmp[UA] + g - ZP, uap);
+        if (C == 0 && c.j >= 1) l4(P.b.tmp[UB] + g - ZP, ubp);
+        if (C != 0 && c.i >= 1) l4(P.b.tmp[UB] + g - NYZ, ubp);
+        if (C != 2 && c.lane == 0 && c.kb >= 1) zk = P.b.tmp[UA][g - 1];
+    }
+    if (C != 2) {
+        const float t = __shfl_up_sync(0xffffffffu, ua[3], 1);
+        if (c.lane != 0) zk = t;
+        if (c.kb == 0) zk = 0.f;
+        uap[0] = zk; uap[1] = ua[0]; uap[2] = ua[1]; uap[3] = ua[2];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        ge[q] += (uap[q] - ua[q]) * P.rdx + (ubp[q] - ub[q]) * P.rdx;
+}
+
+// E part of component C. FIN: the fin of the later step first (gE then carries it).
+// ADD: tmp6..8 accumulate (clear: this step starts the run's sum). MODE bit 0: damping,
+// bit 1: poles.
+template <int C, bool FIN, bool ADD, int MODE>
+__device__ __forceinline__ void a3_e(const Adj3 &P, const A3Cell &c, const float *en_,
+                                     const float *eo_, int64_t rec_comp) {
+    constexpr bool DAMP = (MODE & 1) != 0, PL = (MODE & 2) != 0;
     const int nx = P.nx, ny = P.ny, nz = P.nz, ZP = P.zp;
-    const int lane = threadIdx.x;
-    const int j = blockIdx.y * A3Y + threadIdx.y;
-    const int i = blockIdx.z;
-    const int kb = blockIdx.x * 128 + 4 * lane;
-    const bool act = j < ny && kb < ZP;
-    const uint32_t NYZ = (uint32_t)ny * ZP;
-    const uint32_t g = (uint32_t)i * NYZ + (uint32_t)(j * ZP + kb);
+    const int i = c.i, j = c.j, kb = c.kb;
+    const uint32_t g = c.g, NYZ = (uint32_t)ny * ZP;
     const mtb_adj3d_buffers &B = P.b;
     const float dt = P.dt;
-    float ep[4], epi[4], epj[4], epk = 1.f;
-    ep[0] = ep[1] = ep[2] = ep[3] = 1.f;
-    epi[0] = epi[1] = epi[2] = epi[3] = 1.f;
-    epj[0] = epj[1] = epj[2] = epj[3] = 1.f;
-    if (act) {
-        l4(P.eps + g, ep);
-        if (i + 1 < nx) l4(P.eps + g + NYZ, epi);
-        if (j + 1 < ny) l4(P.eps + g + ZP, epj);
-        if (lane == 31 && kb + 4 < ZP) epk = P.eps[g + 4];
-    }
-    {
-        const float t = __shfl_down_sync(0xffffffffu, ep[0], 1);
-        if (lane != 31) epk = t;
-    }
-    if (!act) return;
+    const bool act = c.act;
     const bool iin = i >= 1 && i <= nx - 2, jin = j >= 1 && j <= ny - 2;
     const bool xok = i <= nx - 2, vyH = j <= ny - 2;
-    float ge[3][4], en[3][4], eo[3][4], gp[6][4];
-    for (int c = 0; c < 3; ++c) {
-        l4(B.g[c] + g, ge[c]);
-        l4(en_ + c * rec_comp + g, en[c]);
-        l4(eo_ + c * rec_comp + g, eo[c]);
+    // first term (psi 6 + 2C, tmp 2C) and second (psi 7 + 2C, tmp 2C + 1) and their axes:
+    // Ex: y, z; Ey: z, x; Ez: x, y
+    float b0, a0, b1 = 1.f, a1 = 0.f, zb[4], za[4];
+    if (C == 0) a3_prof(P, 1, 1, act && jin, j, b0, a0);
+    else a3_prof(P, 0, 1, act && iin, i, b0, a0);
+    if (C == 2) a3_prof(P, 1, 1, act && jin, j, b1, a1);
+    bool zon = false;
+    if (C != 2)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = kb + q;
+            a3_prof(P, 2, 1, act && k >= 1 && k <= nz - 2, k, zb[q], za[q]);
+            zon |= za[q] != 0.f;
+        }
+    // the psi adjoint feeds back only through a: outside the layers it is not needed
+    const bool pA = act && (P.psi_all || (C == 0 ? a0 != 0.f : C == 1 ? zon : a0 != 0.f));
+    const bool pB = act && (P.psi_all || (C == 0 ? zon : C == 1 ? a0 != 0.f : a1 != 0.f));
+    float ep[4], epn[4], ge[4], en[4], eo[4], gs[4], g6[4], g7[4], epk = 1.f;
+    ep[0] = ep[1] = ep[2] = ep[3] = 1.f;
+    epn[0] = epn[1] = epn[2] = epn[3] = 1.f;
+    zz(ge); zz(en); zz(eo); zz(gs); zz(g6); zz(g7);
+    float d1[4] = {1.f, 1.f, 1.f, 1.f}, d2[4] = {dt, dt, dt, dt};
+    if (act) {
+        l4(P.eps + g, ep);
+        if (C == 0 && i + 1 < nx) l4(P.eps + g + NYZ, epn);
+        if (C == 1 && j + 1 < ny) l4(P.eps + g + ZP, epn);
+        if (C == 2 && c.lane == 31 && kb + 4 < ZP) epk = P.eps[g + 4];
+        l4(B.g[C] + g, ge);
+        l4(en_ + C * rec_comp + g, en);
+        l4(eo_ + C * rec_comp + g, eo);
+        if (ADD) l4(B.tmp[6 + C] + g, gs);
+        if (pA) l4(B.g_psi[6 + 2 * C] + g, g6);
+        if (pB) l4(B.g_psi[7 + 2 * C] + g, g7);
+        // conductive damping: E' = d1 E + (d2 curl + s) / eps_c (core/stepper_3d.py:405-437)
+        if (DAMP) { l4(P.dmp[C][0] + g, d1); l4(P.dmp[C][1] + g, d2); }
     }
-    for (int c = 0; c < 6; ++c) l4(B.g_psi[6 + c] + g, gp[c]);
-    // conductive damping: E' = d1 E + (d2 curl + s) / eps_c (core/stepper_3d.py:405-437)
-    const bool damp = P.dmp[0][0] != nullptr;
-    float d1[3][4], d2[3][4];
-    for (int c = 0; c < 3; ++c)
-        for (int q = 0; q < 4; ++q) { d1[c][q] = 1.f; d2[c][q] = dt; }
-    if (damp)
-        for (int c = 0; c < 3; ++c) { l4(P.dmp[c][0] + g, d1[c]); l4(P.dmp[c][1] + g, d2[c]); }
+    if (C == 2) {
+        const float t = __shfl_down_sync(0xffffffffu, ep[0], 1);
+        if (c.lane != 31) epk = t;
+        if (kb + 4 >= ZP) epk = 1.f;
+        epn[0] = ep[1]; epn[1] = ep[2]; epn[2] = ep[3]; epn[3] = epk;
+    }
+    if (FIN) a3_fin<C>(P, c, ge);
+    if (!act) return;
     // dispersive poles (core/stepper_3d.py:295-300, :311-322): P(n+1) = c1 P(n) +
     // c2 P(n-1) + c3 E(n), E' = (d1 (E eps_c + sum P(n)) + d2 curl + s - sum P(n+1)) / eps_c.
     // P(n+1) is the next state's P(n), so gN = d J / d P(n+1) = gPc' - gE' / eps_c, and
     //   d J / d E(n) gains sum c3 gN,  gPc = d1 gE' / eps_c + c1 gN + gPp',  gPp = c2 gN.
-    float pe[3][4];
-    for (int c = 0; c < 3; ++c) zz(pe[c]);
-    if (P.np > 0) {
+    float pe[4];
+    zz(pe);
+    if (PL) {
         const size_t plane = (size_t)nx * NYZ;
-        for (int c = 0; c < 3; ++c) {
-            float ec[4];
-            bool pv[4];
+#pragma unroll 1
+        for (int p = 0; p < P.np; ++p) {
+            float *gc_ = B.g_pol[C][0] + p * plane + g;
+            float *gq_ = B.g_pol[C][1] + p * plane + g;
+            float gpc[4], gpp[4], c3[4];
+            l4(gc_, gpc); l4(gq_, gpp); l4(P.c3[C] + p * plane + g, c3);
+            const float c1 = P.c1[p], c2 = P.c2[p];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int k = kb + q;
-                const float o = c == 0 ? epi[q] : c == 1 ? epj[q] : (q < 3 ? ep[q + 1] : epk);
-                ec[q] = 0.5f * (ep[q] + o);
-                pv[q] = c == 0 ? (xok && k < nz) : c == 1 ? (vyH && k < nz) : (k <= nz - 2);
+                if (!(C == 0 ? (xok && k < nz) : C == 1 ? (vyH && k < nz) : (k <= nz - 2)))
+                    continue;
+                const float ec = 0.5f * (ep[q] + epn[q]);
+                const float gE = ge[q];
+                const float gN = gpc[q] - gE / ec;
+                pe[q] += c3[q] * gN;
+                gpc[q] = d1[q] * gE / ec + c1 * gN + gpp[q];
+                gpp[q] = c2 * gN;
             }
-            for (int p = 0; p < P.np; ++p) {
-                float *gc_ = B.g_pol[c][0] + p * plane + g;
-                float *gq_ = B.g_pol[c][1] + p * plane + g;
-                float gpc[4], gpp[4], c3[4];
-                l4(gc_, gpc); l4(gq_, gpp); l4(P.c3[c] + p * plane + g, c3);
-                const float c1 = P.c1[p], c2 = P.c2[p];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (!pv[q]) continue;
-                    const float gE = ge[c][q];
-                    const float gN = gpc[q] - gE / ec[q];
-                    pe[c][q] += c3[q] * gN;
-                    gpc[q] = d1[c][q] * gE / ec[q] + c1 * gN + gpp[q];
-                    gpp[q] = c2 * gN;
-                }
-                s4(gc_, gpc); s4(gq_, gpp);
-            }
+            s4(gc_, gpc); s4(gq_, gpp);
         }
     }
     // PMC walls (core/stepper_3d.py _term_pmc :99-121): the tangential E on the wall is
     // live, and there the term differentiating along the wall's axis is zero
     const bool iL = iin || (P.pmc & 1), jL = jin || (P.pmc & 2);
-    // E-side profiles (1, 0) on inert nodes
-    const float exb = prof(P.pb[0][1], iin, 1.f, i), exa = prof(P.pa[0][1], iin, 0.f, i);
-    const float eyb = prof(P.pb[1][1], jin, 1.f, j), eya = prof(P.pa[1][1], jin, 0.f, j);
-    float t[9][4];
+    float t0[4], t1[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int k = kb + q;
-        const bool vzE = k < nz, vz = k <= nz - 2, kin = k >= 1 && k <= nz - 2;
-        const bool kL = kin || (P.pmc & 4);
-        const float ezb = prof(P.pb[2][1], kin, 1.f, k), eza = prof(P.pa[2][1], kin, 0.f, k);
-        // Ex: valid i <= nx-2, k < nz; curl on j, k interior
-        {
-            const bool v = xok && vzE, in = v && jL && kL;
-            const float e_x = 0.5f * (ep[q] + epi[q]);
-            const float gE = ge[0][q];
-            t[6][q] = v ? -gE * (en[0][q] - d1[0][q] * eo[0][q]) / e_x : 0.f;
-            const float gc = in ? d2[0][q] * gE / e_x : 0.f;
-            ge[0][q] = v ? d1[0][q] * gE + pe[0][q] : gE;   // d1 gE (+ poles) to E
-            const float g6 = gp[0][q] + gc, g7 = gp[1][q] - gc;
-            const bool u6 = v && jin, u7 = v && kin;
-            gp[0][q] = u6 ? eyb * g6 : gp[0][q];
-            gp[1][q] = u7 ? ezb * g7 : gp[1][q];
-            t[0][q] = u6 ? gc + eya * g6 : 0.f;                    // dy(Hz)
-            t[1][q] = u7 ? -gc + eza * g7 : 0.f;                   // dz(Hy)
-        }
-        // Ey: valid j <= ny-2, k < nz; curl on i, k interior
-        {
-            const bool v = vyH && vzE, in = v && iL && kL;
-            const float e_y = 0.5f * (ep[q] + epj[q]);
-            const float gE = ge[1][q];
-            t[7][q] = v ? -gE * (en[1][q] - d1[1][q] * eo[1][q]) / e_y : 0.f;
-            const float gc = in ? d2[1][q] * gE / e_y : 0.f;
-            ge[1][q] = v ? d1[1][q] * gE + pe[1][q] : gE;   // d1 gE (+ poles) to E
-            const float g8 = gp[2][q] + gc, g9 = gp[3][q] - gc;
-            const bool u8 = v && kin, u9 = v && iin;
-            gp[2][q] = u8 ? ezb * g8 : gp[2][q];
-            gp[3][q] = u9 ? exb * g9 : gp[3][q];
-            t[2][q] = u8 ? gc + eza * g8 : 0.f;                    // dz(Hx)
-            t[3][q] = u9 ? -gc + exa * g9 : 0.f;                   // dx(Hz)
-        }
-        // Ez: valid k <= nz-2; curl on i, j interior
-        {
-            const bool v = vz, in = v && iL && jL;
-            const float e_z = 0.5f * (ep[q] + ((q < 3) ? ep[q + 1] : epk));
-            const float gE = ge[2][q];
-            t[8][q] = v ? -gE * (en[2][q] - d1[2][q] * eo[2][q]) / e_z : 0.f;
-            const float gc = in ? d2[2][q] * gE / e_z : 0.f;
-            ge[2][q] = v ? d1[2][q] * gE + pe[2][q] : gE;   // d1 gE (+ poles) to E
-            const float g10 = gp[4][q] + gc, g11 = gp[5][q] - gc;
-            const bool u10 = v && iin, u11 = v && jin;
-            gp[4][q] = u10 ? exb * g10 : gp[4][q];
-            gp[5][q] = u11 ? eyb * g11 : gp[5][q];
-            t[4][q] = u10 ? gc + exa * g10 : 0.f;                  // dx(Hy)
-            t[5][q] = u11 ? -gc + eya * g11 : 0.f;                 // dy(Hx)
-        }
+        const bool kin = k >= 1 && k <= nz - 2, kL = kin || (P.pmc & 4);
+        const bool v = C == 0 ? (xok && k < nz) : C == 1 ? (vyH && k < nz) : (k <= nz - 2);
+        const bool in = v && (C == 0 ? jL && kL : C == 1 ? iL && kL : iL && jL);
+        const float ec = 0.5f * (ep[q] + epn[q]);
+        const float gE = ge[q];
+        gs[q] = v ? gs[q] - gE * (en[q] - d1[q] * eo[q]) : gs[q];
+        const float gc = in ? d2[q] * gE / ec : 0.f;
+        if (DAMP || PL) ge[q] = v ? d1[q] * gE + pe[q] : gE;   // d1 gE (+ poles) to E
+        const bool uA = v && (C == 0 ? jin : C == 1 ? kin : iin);
+        const bool uB = v && (C == 0 ? kin : C == 1 ? iin : jin);
+        const float bA = C == 1 ? zb[q] : b0, aA = C == 1 ? za[q] : a0;
+        const float bB = C == 0 ? zb[q] : C == 1 ? b0 : b1;
+        const float aB = C == 0 ? za[q] : C == 1 ? a0 : a1;
+        const float gA = g6[q] + gc, gB = g7[q] - gc;
+        g6[q] = uA ? bA * gA : g6[q];
+        g7[q] = uB ? bB * gB : g7[q];
+        t0[q] = uA ? gc + aA * gA : 0.f;
+        t1[q] = uB ? -gc + aB * gB : 0.f;
     }
-    for (int c = 0; c < 6; ++c) s4(B.g_psi[6 + c] + g, gp[c]);
-    for (int c = 0; c < 9; ++c) s4(B.tmp[c] + g, t[c]);
-    if (damp || P.np > 0)
-        for (int c = 0; c < 3; ++c) s4(B.g[c] + g, ge[c]);
+    if (FIN || DAMP || PL) s4(B.g[C] + g, ge);
+    s4(B.tmp[6 + C] + g, gs);
+    s4(B.tmp[2 * C] + g, t0);
+    s4(B.tmp[2 * C + 1] + g, t1);
+    if (pA) s4(B.g_psi[6 + 2 * C] + g, g6);
+    if (pB) s4(B.g_psi[7 + 2 * C] + g, g7);
 }
 
-__global__ void __launch_bounds__(32 * A3Y) k_adj3_h(const __grid_constant__ Adj3 P) {
+// The E part of one step, after the fin of the step that follows it when FIN. What
+// bounds it: L2 / HBM bytes (18 floats a cell without layers).
+template <bool FIN, int MODE>
+__global__ void __launch_bounds__(3 * A3_T, 2) k_adj3_fe(const __grid_constant__ Adj3 P,
+                                                        const float *__restrict__ en,
+                                                        const float *__restrict__ eo,
+                                                        int64_t rec_comp) {
+    const A3Cell c(P);
+    if (threadIdx.y == 0) a3_e<0, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
+    else if (threadIdx.y == 1) a3_e<1, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
+    else a3_e<2, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
+}
+
+// H part of component C.
+template <int C>
+__device__ __forceinline__ void a3_h(const Adj3 &P, const A3Cell &c) {
+    // transposed differences of the E part's H derivatives, in the order
+    // Hx: 2 (z), 5 (y); Hy: 1 (z), 4 (x); Hz: 0 (y), 3 (x)
+    constexpr int TA = C == 0 ? 2 : C == 1 ? 1 : 0, TB = C == 0 ? 5 : C == 1 ? 4 : 3;
     const int nx = P.nx, ny = P.ny, nz = P.nz, ZP = P.zp;
-    const int lane = threadIdx.x;
-    const int j = blockIdx.y * A3Y + threadIdx.y;
-    const int i = blockIdx.z;
-    const int kb = blockIdx.x * 128 + 4 * lane;
-    const bool act = j < ny && kb < ZP;
-    const uint32_t NYZ = (uint32_t)ny * ZP;
-    const uint32_t g = (uint32_t)i * NYZ + (uint32_t)(j * ZP + kb);
+    const int i = c.i, j = c.j, kb = c.kb;
+    const uint32_t g = c.g, NYZ = (uint32_t)ny * ZP;
     const mtb_adj3d_buffers &B = P.b;
     const float dt = P.dt, rdx = P.rdx;
-    // own and +1 neighbours of the E-kernel adjoints
-    float t0[4], t0j[4], t3[4], t3i[4], t1[4], t4[4], t4i[4], t2[4], t5[4], t5j[4];
-    float t1k = 0.f, t2k = 0.f;
-    zz(t0); zz(t0j); zz(t3); zz(t3i); zz(t1); zz(t4); zz(t4i); zz(t2); zz(t5); zz(t5j);
+    const bool act = c.act, xok = i <= nx - 2, vyH = j <= ny - 2;
+    // psi 2C (tmp 9 + 2C) and psi 2C + 1 (tmp 10 + 2C): Hx: y, z; Hy: z, x; Hz: x, y
+    float b0, a0, b1 = 1.f, a1 = 0.f, zb[4], za[4];
+    if (C == 0) a3_prof(P, 1, 0, act && vyH, j, b0, a0);
+    else a3_prof(P, 0, 0, act && xok, i, b0, a0);
+    if (C == 2) a3_prof(P, 1, 0, act && vyH, j, b1, a1);
+    bool zon = false;
+    if (C != 2)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            a3_prof(P, 2, 0, act && kb + q <= nz - 2, kb + q, zb[q], za[q]);
+            zon |= za[q] != 0.f;
+        }
+    const bool pA = act && (P.psi_all || (C == 0 ? a0 != 0.f : C == 1 ? zon : a0 != 0.f));
+    const bool pB = act && (P.psi_all || (C == 0 ? zon : C == 1 ? a0 != 0.f : a1 != 0.f));
+    float ta[4], tan_[4], tb[4], tbn[4], gh[4], g0[4], g1[4], zk = 0.f;
+    zz(ta); zz(tan_); zz(tb); zz(tbn); zz(gh); zz(g0); zz(g1);
+    float h1[4] = {1.f, 1.f, 1.f, 1.f}, h2[4] = {dt, dt, dt, dt};
+    const bool damp = P.dmp[3][0] != nullptr;
     if (act) {
-        l4(B.tmp[0] + g, t0); l4(B.tmp[1] + g, t1); l4(B.tmp[2] + g, t2);
-        l4(B.tmp[3] + g, t3); l4(B.tmp[4] + g, t4); l4(B.tmp[5] + g, t5);
-        if (j + 1 < ny) { l4(B.tmp[0] + g + ZP, t0j); l4(B.tmp[5] + g + ZP, t5j); }
-        if (i + 1 < nx) { l4(B.tmp[3] + g + NYZ, t3i); l4(B.tmp[4] + g + NYZ, t4i); }
-        if (lane == 31 && kb + 4 < ZP) { t1k = B.tmp[1][g + 4]; t2k = B.tmp[2][g + 4]; }
+        l4(B.tmp[TA] + g, ta);
+        l4(B.tmp[TB] + g, tb);
+        if (C == 2 && j + 1 < ny) l4(B.tmp[TA] + g + ZP, tan_);
+        if (C == 0 && j + 1 < ny) l4(B.tmp[TB] + g + ZP, tbn);
+        if (C != 0 && i + 1 < nx) l4(B.tmp[TB] + g + NYZ, tbn);
+        if (C != 2 && c.lane == 31 && kb + 4 < ZP) zk = B.tmp[TA][g + 4];
+        l4(B.g[3 + C] + g, gh);
+        if (pA) l4(B.g_psi[2 * C] + g, g0);
+        if (pB) l4(B.g_psi[2 * C + 1] + g, g1);
+        // conductive damping: H' = d1 H - d2 curl (core/stepper_3d.py:375-393)
+        if (damp) { l4(P.dmp[3 + C][0] + g, h1); l4(P.dmp[3 + C][1] + g, h2); }
     }
-    {
-        const float a = __shfl_down_sync(0xffffffffu, t1[0], 1);
-        const float b = __shfl_down_sync(0xffffffffu, t2[0], 1);
-        if (lane != 31) { t1k = a; t2k = b; }
+    if (C != 2) {
+        const float t = __shfl_down_sync(0xffffffffu, ta[0], 1);
+        if (c.lane != 31) zk = t;
+        if (kb + 4 >= ZP) zk = 0.f;
+        tan_[0] = ta[1]; tan_[1] = ta[2]; tan_[2] = ta[3]; tan_[3] = zk;
     }
     if (!act) return;
-    const bool xok = i <= nx - 2, vyH = j <= ny - 2;
-    float gh[3][4], gp[6][4];
-    for (int c = 0; c < 3; ++c) l4(B.g[3 + c] + g, gh[c]);
-    for (int c = 0; c < 6; ++c) l4(B.g_psi[c] + g, gp[c]);
-    const float hxb = prof(P.pb[0][0], xok, 1.f, i), hxa = prof(P.pa[0][0], xok, 0.f, i);
-    const float hyb = prof(P.pb[1][0], vyH, 1.f, j), hya = prof(P.pa[1][0], vyH, 0.f, j);
-    // conductive damping: H' = d1 H - d2 curl (core/stepper_3d.py:375-393)
-    float h1[3][4], h2[3][4];
-    for (int c = 0; c < 3; ++c)
-        for (int q = 0; q < 4; ++q) { h1[c][q] = 1.f; h2[c][q] = dt; }
-    if (P.dmp[3][0])
-        for (int c = 0; c < 3; ++c) { l4(P.dmp[3 + c][0] + g, h1[c]); l4(P.dmp[3 + c][1] + g, h2[c]); }
-    float u[6][4];
+    float u0[4], u1[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int k = kb + q;
-        const bool vz = k <= nz - 2, vzE = k < nz;
-        const float hzb = prof(P.pb[2][0], vz, 1.f, k), hza = prof(P.pa[2][0], vz, 0.f, k);
-        const float t1n = (q < 3) ? t1[q + 1] : t1k;
-        const float t2n = (q < 3) ? t2[q + 1] : t2k;
-        // transposed differences of the E kernel's H derivatives
-        const float gx = gh[0][q] + (t2[q] - t2n) * rdx + (t5[q] - t5j[q]) * rdx;
-        const float gy = gh[1][q] + (t1[q] - t1n) * rdx + (t4[q] - t4i[q]) * rdx;
-        const float gz = gh[2][q] + (t0[q] - t0j[q]) * rdx + (t3[q] - t3i[q]) * rdx;
-        // Hx -= dt ((dy + psi0') - (dz + psi1')): valid j <= ny-2, k <= nz-2
-        {
-            const bool v = vyH && vz;
-            const float c0 = -h2[0][q] * gx, c1 = h2[0][q] * gx;
-            const float g0 = gp[0][q] + c0, g1 = gp[1][q] + c1;
-            u[0][q] = v ? c0 + hya * g0 : 0.f;                     // dy(Ez)
-            u[1][q] = v ? c1 + hza * g1 : 0.f;                     // dz(Ey)
-            gp[0][q] = v ? hyb * g0 : gp[0][q];
-            gp[1][q] = v ? hzb * g1 : gp[1][q];
-            gh[0][q] = v ? h1[0][q] * gx : gx;
-        }
-        // Hy -= dt ((dz + psi2') - (dx + psi3')): valid i <= nx-2, k <= nz-2
-        {
-            const bool v = xok && vz;
-            const float c2 = -h2[1][q] * gy, c3 = h2[1][q] * gy;
-            const float g2 = gp[2][q] + c2, g3 = gp[3][q] + c3;
-            u[2][q] = v ? c2 + hza * g2 : 0.f;                     // dz(Ex)
-            u[3][q] = v ? c3 + hxa * g3 : 0.f;                     // dx(Ez)
-            gp[2][q] = v ? hzb * g2 : gp[2][q];
-            gp[3][q] = v ? hxb * g3 : gp[3][q];
-            gh[1][q] = v ? h1[1][q] * gy : gy;
-        }
-        // Hz -= dt ((dx + psi4') - (dy + psi5')): valid i <= nx-2, j <= ny-2, k < nz
-        {
-            const bool v = xok && vyH && vzE;
-            const float c4 = -h2[2][q] * gz, c5 = h2[2][q] * gz;
-            const float g4 = gp[4][q] + c4, g5 = gp[5][q] + c5;
-            u[4][q] = v ? c4 + hxa * g4 : 0.f;                     // dx(Ey)
-            u[5][q] = v ? c5 + hya * g5 : 0.f;                     // dy(Ex)
-            gp[4][q] = v ? hxb * g4 : gp[4][q];
-            gp[5][q] = v ? hyb * g5 : gp[5][q];
-            gh[2][q] = v ? h1[2][q] * gz : gz;
-        }
+        const bool vz = k <= nz - 2;
+        const bool v = C == 0 ? (vyH && vz) : C == 1 ? (xok && vz) : (xok && vyH && k < nz);
+        const float gx = gh[q] + (ta[q] - tan_[q]) * rdx + (tb[q] - tbn[q]) * rdx;
+        // H -= dt ((A + psi A') - (B + psi B'))
+        const float bA = C == 1 ? zb[q] : b0, aA = C == 1 ? za[q] : a0;
+        const float bB = C == 0 ? zb[q] : C == 1 ? b0 : b1;
+        const float aB = C == 0 ? za[q] : C == 1 ? a0 : a1;
+        const float cA = -h2[q] * gx, cB = h2[q] * gx;
+        const float gA = g0[q] + cA, gB = g1[q] + cB;
+        u0[q] = v ? cA + aA * gA : 0.f;
+        u1[q] = v ? cB + aB * gB : 0.f;
+        g0[q] = v ? bA * gA : g0[q];
+        g1[q] = v ? bB * gB : g1[q];
+        gh[q] = v ? h1[q] * gx : gx;
     }
-    for (int c = 0; c < 3; ++c) s4(B.g[3 + c] + g, gh[c]);
-    for (int c = 0; c < 6; ++c) s4(B.g_psi[c] + g, gp[c]);
-    for (int c = 0; c < 6; ++c) s4(B.tmp[9 + c] + g, u[c]);
+    s4(B.g[3 + C] + g, gh);
+    s4(B.tmp[9 + 2 * C] + g, u0);
+    s4(B.tmp[10 + 2 * C] + g, u1);
+    if (pA) s4(B.g_psi[2 * C] + g, g0);
+    if (pB) s4(B.g_psi[2 * C + 1] + g, g1);
 }
 
-__global__ void __launch_bounds__(32 * A3Y) k_adj3_fin(const __grid_constant__ Adj3 P) {
-    const int nx = P.nx, ny = P.ny, nz = P.nz, ZP = P.zp;
-    const int lane = threadIdx.x;
-    const int j = blockIdx.y * A3Y + threadIdx.y;
-    const int i = blockIdx.z;
-    const int kb = blockIdx.x * 128 + 4 * lane;
-    const bool act = j < ny && kb < ZP;
-    const uint32_t NYZ = (uint32_t)ny * ZP;
-    const uint32_t g = (uint32_t)i * NYZ + (uint32_t)(j * ZP + kb);
+__global__ void __launch_bounds__(3 * A3_T, 2) k_adj3_h(const __grid_constant__ Adj3 P) {
+    const A3Cell c(P);
+    if (threadIdx.y == 0) a3_h<0>(P, c);
+    else if (threadIdx.y == 1) a3_h<1>(P, c);
+    else a3_h<2>(P, c);
+}
+
+// The last step's fin (gE only).
+__global__ void __launch_bounds__(3 * A3_T) k_adj3_fin(const __grid_constant__ Adj3 P) {
+    const A3Cell c(P);
+    const int C = threadIdx.y;
+    float ge[4];
+    zz(ge);
+    if (c.act) l4(P.b.g[C] + c.g, ge);
+    if (C == 0) a3_fin<0>(P, c, ge);
+    else if (C == 1) a3_fin<1>(P, c, ge);
+    else a3_fin<2>(P, c, ge);
+    if (c.act) s4(P.b.g[C] + c.g, ge);
+}
+
+// g_eps += the run's sums of each component's eps_c adjoint, divided by eps_c, at the two
+// cells of its Yee average.
+__global__ void __launch_bounds__(A3_T) k_adj3_eps(const __grid_constant__ Adj3 P) {
+    const A3Cell c(P);
+    if (!c.act) return;
+    const int i = c.i, j = c.j, ZP = P.zp;
+    const uint32_t g = c.g, NYZ = (uint32_t)P.ny * ZP;
     const mtb_adj3d_buffers &B = P.b;
-    const float rdx = P.rdx;
-    // own and -1 neighbours of the H-kernel adjoints and of the eps parts
-    float u9[4], u9j[4], u10[4], u11[4], u12[4], u12i[4], u13[4], u13i[4], u14[4], u14j[4];
-    float t6[4], t6i[4], t7[4], t7j[4], t8[4];
-    float u10k = 0.f, u11k = 0.f, t8k = 0.f;
-    zz(u9); zz(u9j); zz(u10); zz(u11); zz(u12); zz(u12i); zz(u13); zz(u13i); zz(u14); zz(u14j);
-    zz(t6); zz(t6i); zz(t7); zz(t7j); zz(t8);
-    if (act) {
-        l4(B.tmp[9] + g, u9); l4(B.tmp[10] + g, u10); l4(B.tmp[11] + g, u11);
-        l4(B.tmp[12] + g, u12); l4(B.tmp[13] + g, u13); l4(B.tmp[14] + g, u14);
-        l4(B.tmp[6] + g, t6); l4(B.tmp[7] + g, t7); l4(B.tmp[8] + g, t8);
-        if (j >= 1) { l4(B.tmp[9] + g - ZP, u9j); l4(B.tmp[14] + g - ZP, u14j); l4(B.tmp[7] + g - ZP, t7j); }
-        if (i >= 1) { l4(B.tmp[12] + g - NYZ, u12i); l4(B.tmp[13] + g - NYZ, u13i); l4(B.tmp[6] + g - NYZ, t6i); }
-        if (lane == 0 && kb >= 1) { u10k = B.tmp[10][g - 1]; u11k = B.tmp[11][g - 1]; t8k = B.tmp[8][g - 1]; }
-    }
-    {
-        const float a = __shfl_up_sync(0xffffffffu, u10[3], 1);
-        const float b = __shfl_up_sync(0xffffffffu, u11[3], 1);
-        const float c = __shfl_up_sync(0xffffffffu, t8[3], 1);
-        if (lane != 0) { u10k = a; u11k = b; t8k = c; }
-    }
-    if (!act) return;
-    float ge[3][4], geps[4];
-    for (int c = 0; c < 3; ++c) l4(B.g[c] + g, ge[c]);
-    l4(B.g_eps + g, geps);
+    float e[4], ei[4], eim[4], ej[4], ejm[4], t6[4], t6i[4], t7[4], t7j[4], t8[4], ge[4];
+    zz(t6i); zz(t7j);
+    l4(P.eps + g, e);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ei[q] = eim[q] = ej[q] = ejm[q] = e[q];
+    l4(B.tmp[6] + g, t6); l4(B.tmp[7] + g, t7); l4(B.tmp[8] + g, t8);
+    if (i + 1 < P.nx) l4(P.eps + g + NYZ, ei);
+    if (j + 1 < P.ny) l4(P.eps + g + ZP, ej);
+    if (i >= 1) { l4(P.eps + g - NYZ, eim); l4(B.tmp[6] + g - NYZ, t6i); }
+    if (j >= 1) { l4(P.eps + g - ZP, ejm); l4(B.tmp[7] + g - ZP, t7j); }
+    const float em = c.kb >= 1 ? P.eps[g - 1] : 1.f, t8m = c.kb >= 1 ? B.tmp[8][g - 1] : 0.f;
+    const float ekp = c.kb + 4 < ZP ? P.eps[g + 4] : 1.f;
+    l4(B.g_eps + g, ge);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const int k = kb + q;
-        const float u10m = (q == 0) ? u10k : u10[q - 1];
-        const float u11m = (q == 0) ? u11k : u11[q - 1];
-        const float t8m = (q == 0) ? t8k : t8[q - 1];
-        // Ex: in dz(Ex) of Hy (k+1 - k) and dy(Ex) of Hz (j+1 - j)
-        ge[0][q] += (u11m - u11[q]) * rdx + (u14j[q] - u14[q]) * rdx;
-        // Ey: in dz(Ey) of Hx and dx(Ey) of Hz
-        ge[1][q] += (u10m - u10[q]) * rdx + (u13i[q] - u13[q]) * rdx;
-        // Ez: in dy(Ez) of Hx and dx(Ez) of Hy
-        ge[2][q] += (u9j[q] - u9[q]) * rdx + (u12i[q] - u12[q]) * rdx;
-        if (k < nz)
-            geps[q] += 0.5f * (t6[q] + t6i[q]) + 0.5f * (t7[q] + t7j[q]) + 0.5f * (t8[q] + t8m);
+        const int k = c.kb + q;
+        if (k >= P.nz) continue;
+        const float ek = q < 3 ? e[q + 1] : ekp, ekm = q > 0 ? e[q - 1] : em;
+        const float tk = q > 0 ? t8[q - 1] : t8m;
+        // a sum is zero outside its component's cells; the average there may be with padding
+        const float x = t6[q] / (0.5f * (e[q] + ei[q])) + t6i[q] / (0.5f * (eim[q] + e[q]));
+        const float y = t7[q] / (0.5f * (e[q] + ej[q])) + t7j[q] / (0.5f * (ejm[q] + e[q]));
+        const float z = (k <= P.nz - 2 ? t8[q] / (0.5f * (e[q] + ek)) : 0.f) +
+                        (k >= 1 ? tk / (0.5f * (ekm + e[q])) : 0.f);
+        ge[q] += 0.5f * x + 0.5f * y + 0.5f * z;
     }
-    for (int c = 0; c < 3; ++c) s4(B.g[c] + g, ge[c]);
-    s4(B.g_eps + g, geps);
+    s4(B.g_eps + g, ge);
 }
 
 }  // namespace mtb
@@ -412,8 +452,7 @@ int mtb_yee3d_adjoint_create(const mtb_yee3d_struct *s, const mtb_adj3d_buffers 
     if (S.pmc_axes & ~7) return fail(MTB_INVALID_ARG, "3D adjoint: pmc_axes %d", S.pmc_axes);
     if (S.nx < 3 || S.ny < 3 || S.nz < 3 || S.zpitch < S.nz || (S.zpitch & 3))
         return fail(MTB_INVALID_ARG, "3D adjoint: bad grid");
-    if ((int64_t)S.nx * S.ny * S.zpitch >= (1LL << 31) || S.nx > 65535 ||
-        (S.ny + A3Y - 1) / A3Y > 65535)
+    if ((int64_t)S.nx * S.ny * S.zpitch >= (1LL << 31) || S.nx > 65535 || S.ny > 65535 * 8)
         return fail(MTB_UNSUPPORTED, "3D adjoint: grid too large");
     auto bad = [](const void *p) { return !p || (reinterpret_cast<uintptr_t>(p) & 15); };
     for (int c = 0; c < 6; ++c)
@@ -448,6 +487,7 @@ int mtb_yee3d_adjoint_create(const mtb_yee3d_struct *s, const mtb_adj3d_buffers 
         for (int h = 0; h < 2; ++h) A.dmp[c][h] = S.damp[c][h];
     A.np = S.n_poles;
     A.pmc = S.pmc_axes;
+    A.psi_all = 1;
     for (int c = 0; c < 3; ++c) A.c3[c] = S.n_poles ? S.pol_c3[c] : nullptr;
     for (int p = 0; p < MTB_MAX_POLES; ++p) {
         A.c1[p] = p < S.n_poles ? S.pol_c1[p] : 0.f;
@@ -510,26 +550,50 @@ int mtb_yee3d_adjoint_run(mtb_yee3d_adjoint *p, int64_t t0, int32_t k, const flo
                                      sizeof(float) * (size_t)p->dft.slot_elems * k, st));
     }
     const Adj3 &A = p->a;
-    const dim3 blk(32, A3Y);
-    const dim3 grid((A.zp + 127) / 128, (A.ny + A3Y - 1) / A3Y, A.nx);
-    for (int q = k - 1; q >= 0; --q) {
+    const dim3 blk(A3_T, 3);
+    const dim3 grid((unsigned)(((int64_t)A.ny * (A.zp / 4) + A3_T - 1) / A3_T), A.nx);
+    const int mode = (A.dmp[0][0] ? 1 : 0) | (A.np > 0 ? 2 : 0);
+    auto inject = [&](int q) -> int {
+        if (p->n_samples == 0) return MTB_OK;
         const float *radj = p->dft.ring_d.as<float>() + (size_t)q * p->dft.slot_elems;
-        if (p->n_samples > 0) {
-            k_adj3_inject<<<(unsigned)((p->n_samples + 255) / 256), 256, 0, st>>>(
-                p->s_d.as<mtb_yee3d_struct>(), p->pstart_d.as<int64_t>(), p->n_planes, radj, A.b);
-            MTB_CHECK_LAUNCH();
-            ++p->last_launches;
-        }
+        k_adj3_inject<<<(unsigned)((p->n_samples + 255) / 256), 256, 0, st>>>(
+            p->s_d.as<mtb_yee3d_struct>(), p->pstart_d.as<int64_t>(), p->n_planes, radj, A.b);
+        MTB_CHECK_LAUNCH();
+        ++p->last_launches;
+        return MTB_OK;
+    };
+    if ((rc = inject(k - 1))) return rc;
+    for (int q = k - 1; q >= 0; --q) {
         const float *en = rec + (size_t)(q + 1) * rec_slot_stride;
         const float *eo = rec + (size_t)q * rec_slot_stride;
-        k_adj3_e<<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride);
+        const bool fin = q < k - 1;
+        switch (mode + (fin ? 4 : 0)) {
+            case 0: k_adj3_fe<false, 0><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 1: k_adj3_fe<false, 1><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 2: k_adj3_fe<false, 2><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 3: k_adj3_fe<false, 3><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 4: k_adj3_fe<true, 0><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 5: k_adj3_fe<true, 1><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            case 6: k_adj3_fe<true, 2><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+            default: k_adj3_fe<true, 3><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
+        }
         MTB_CHECK_LAUNCH();
         k_adj3_h<<<grid, blk, 0, st>>>(A);
         MTB_CHECK_LAUNCH();
-        k_adj3_fin<<<grid, blk, 0, st>>>(A);
-        MTB_CHECK_LAUNCH();
-        p->last_launches += 3;
+        p->last_launches += 2;
+        if (q > 0 && (rc = inject(q - 1))) return rc;    // before the fin + E launch of q - 1
     }
+    k_adj3_fin<<<grid, blk, 0, st>>>(A);
+    MTB_CHECK_LAUNCH();
+    k_adj3_eps<<<grid, A3_T, 0, st>>>(A);
+    MTB_CHECK_LAUNCH();
+    p->last_launches += 2;
+    return MTB_OK;
+}
+
+int mtb_yee3d_adjoint_psi_layers(mtb_yee3d_adjoint *p, int32_t only_layers) {
+    if (!p) return fail(MTB_INVALID_ARG, "3D adjoint plan is null");
+    p->a.psi_all = only_layers ? 0 : 1;
     return MTB_OK;
 }
 

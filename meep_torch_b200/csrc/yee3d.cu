@@ -407,21 +407,26 @@ __global__ void __launch_bounds__(32 * NZW * (TY3 + 2)) k_yee3d_step(
 }
 
 // ---------------------------------------------------------------- split H / E kernels
-// Streaming variant: one kernel advances H, a second E. A thread updates one
-// float4 of z (4 cells) of one (i, j) row; a block is 32 x 8 threads = 128 z
-// x 8 y of one x plane. Neighbours in y and x come from L1/L2 (the blocks of
-// planes i and i+1 run concurrently), z+-1 from a warp shuffle.
-//  * Every load a thread needs is issued before the first use of any: the
-//    CPML memory is gated by the plan's band limits (geometry), not by the
-//    loaded profile values, so a cell costs one memory round trip.
-//  * The arithmetic is uniform across lanes: outside the layers the CPML
-//    terms run with (b, a) = (1, 0) on psi = 0, which is the reference's own
-//    arithmetic there, and the edge rules are selects, so a warp that holds
-//    both layer and interior cells does not diverge.
-//  * All pointers of one parity are resolved on the host into a by-value
-//    parameter block (no pointer loads in the kernel).
+// Streaming variant: one kernel advances H, a second E. A thread updates one float4 of
+// z (4 cells) of one component: threadIdx.y is the component, threadIdx.x one of S3_T
+// consecutive float4s of the x plane blockIdx.y, counted through the rows (so no lane
+// idles past a row's end, whatever zpitch).
+//  * What bounds it: memory latency. One thread per cell for all three components held
+//    104-158 registers, 8-16 warps an SM, and a cell's whole chain of loads was exposed
+//    (E with a pole: 44.9 us on 128 x 112 x 100, 3.0 TB/s of its L2 traffic). Split by
+//    component a thread has a third of the loads and registers, so three times the warps
+//    hide them; the three components of a float4 share their block, so what two of them
+//    read comes from L1.
+//  * Every load a thread needs is issued before the first use of any: the CPML memory is
+//    gated by the plan's band limits (geometry), not by the loaded profile values.
+//  * The arithmetic is uniform across lanes: outside the layers the CPML terms run with
+//    (b, a) = (1, 0) on psi = 0, which is the reference's own arithmetic there, and the
+//    edge rules are selects, so a warp that holds both layer and interior cells does not
+//    diverge.
+//  * All pointers of one parity are resolved on the host into a by-value parameter block
+//    (no pointer loads in the kernel).
 // DRAM traffic is ~76 B per cell and step plus the CPML memory in the layers.
-constexpr int SPLIT_Y = 8;
+constexpr int S3_T = 128;
 
 // Index k of an axis lies in a CPML band iff k < lo or k >= hi. Superset of
 // the profile's active nodes; psi is loaded / stored there and updated with
@@ -520,135 +525,136 @@ __device__ __forceinline__ void ldg4v(const float *p, float (&v)[4]) {
 }
 __device__ __forceinline__ void one4(float (&v)[4]) { v[0] = v[1] = v[2] = v[3] = 1.f; }
 
-// H(n+1/2) from E(n): core/stepper_3d.py:367-393; DAMP: H' = d1 H - d2 curl
-template <bool DAMP>
-__global__ void __launch_bounds__(32 * SPLIT_Y, 2) k_yee3d_h(const __grid_constant__ Split3 P,
-                                                             int i0) {
+// A thread's float4 in the split kernels: plane i, row j, columns kb .. kb+3, box index g.
+struct S3Cell {
+    int i, j, kb;
+    uint32_t g;
+    bool act;
+    __device__ __forceinline__ S3Cell(const Split3 &P, int i_) {
+        const uint32_t zq = (uint32_t)P.zp >> 2;
+        const uint32_t q = blockIdx.x * (uint32_t)S3_T + threadIdx.x;
+        act = q < (uint32_t)P.ny * zq;               // box < 2^31 elements (plan check)
+        i = i_;
+        j = (int)(q / zq);
+        kb = 4 * (int)(q - (uint32_t)j * zq);
+        g = (uint32_t)i * ((uint32_t)P.ny * P.zp) + 4u * q;
+    }
+};
+
+// One CPML-stretched derivative per cell of a float4, t = d + q with d = (hi - lo) / dx
+// and q = b psi + a d, psi replaced by q where the cell is valid. On z the profile varies
+// over the float4 (bv, av per cell), on x and y it is one pair.
+__device__ __forceinline__ float s3_term(float hi, float lo, float rdx, float b, float a,
+                                         float &psi, bool v) {
+    float q;
+    const float t = y3_s(y3_d(hi, lo, rdx), b, a, psi, q);
+    psi = v ? q : psi;
+    return t;
+}
+// z profile (b, a) of cell k, (1, 0) where it is not applied
+__device__ __forceinline__ void s3_zprof(const float *pb, const float *pa, bool on, int k,
+                                         float &b, float &a) {
+    b = on ? __ldg(pb + k) : 1.f;
+    a = on ? __ldg(pa + k) : 0.f;
+}
+
+// H(n+1/2) of component C from E(n): core/stepper_3d.py:367-393; DAMP: H' = d1 H - d2 curl
+template <int C, bool DAMP>
+__device__ __forceinline__ void s3_h(const Split3 &P, const S3Cell &c) {
     const int nx = P.nx, ny = P.ny, nz = P.nz, ZP = P.zp;
-    const int lane = threadIdx.x;
-    const int j = blockIdx.y * SPLIT_Y + threadIdx.y;
-    const int i = i0 + blockIdx.z;
-    const int kb = blockIdx.x * 128 + 4 * lane;
-    const bool act = j < ny && kb < ZP;
-    const uint32_t NYZ = (uint32_t)ny * ZP;       // box < 2^31 elements (plan check)
-    const uint32_t g = (uint32_t)i * NYZ + (uint32_t)(j * ZP + kb);
-    const float dt = P.dt, rdx = P.rdx;
-    const bool xok = i <= nx - 2, vyH = j <= ny - 2;
+    const int i = c.i, j = c.j, kb = c.kb;
+    const uint32_t g = c.g, NYZ = (uint32_t)ny * ZP;
+    const float rdx = P.rdx;
+    const bool act = c.act, xok = i <= nx - 2, vyH = j <= ny - 2;
     const bool bx = xok && inband(P.B, 0, 0, i), by = vyH && inband(P.B, 1, 0, j);
     bool bz = false;
 #pragma unroll
     for (int q = 0; q < 4; ++q) bz |= kb + q <= nz - 2 && inband(P.B, 2, 0, kb + q);
-    float ex[4], ey[4], ez[4], ezj[4], exj[4], ezi[4], eyi[4], hx[4], hy[4], hz[4];
-    float p0[4], p1[4], p2[4], p3[4], p4[4], p5[4];
-    float eyk = 0.f, exk = 0.f;
-    z4(ex); z4(ey); z4(ez); z4(ezj); z4(exj); z4(ezi); z4(eyi); z4(hx); z4(hy); z4(hz);
-    z4(p0); z4(p1); z4(p2); z4(p3); z4(p4); z4(p5);
+    // Hx: dy Ez (psi 0), dz Ey (psi 1); Hy: dz Ex (psi 2), dx Ez (psi 3);
+    // Hz: dx Ey (psi 4), dy Ex (psi 5)
+    constexpr int FA = C == 0 ? 2 : C == 1 ? 0 : 1;      // first term's E component
+    constexpr int FB = C == 0 ? 1 : C == 1 ? 2 : 0;
+    constexpr int AA = C == 0 ? 1 : C == 1 ? 2 : 0;      // its axis (0 x, 1 y, 2 z)
+    constexpr int AB = C == 0 ? 2 : C == 1 ? 0 : 1;
+    const bool pa_on = C == 0 ? by : C == 1 ? (xok && bz) : (vyH && bx);
+    const bool pb_on = C == 0 ? (vyH && bz) : C == 1 ? bx : (xok && by);
+    float fa[4], fan[4], fb[4], fbn[4], h[4], pa[4], pb[4];
+    z4(fa); z4(fan); z4(fb); z4(fbn); z4(h); z4(pa); z4(pb);
+    float zk = 0.f;                                       // E(k+1) of q = 3
     if (act) {
-        ldg4v(P.e[0] + g, ex); ldg4v(P.e[1] + g, ey); ldg4v(P.e[2] + g, ez);
-        if (j + 1 < ny) { ldg4v(P.e[2] + g + ZP, ezj); ldg4v(P.e[0] + g + ZP, exj); }
-        if (i + 1 < nx) { ldg4v(P.e[2] + g + NYZ, ezi); ldg4v(P.e[1] + g + NYZ, eyi); }
-        if (lane == 31 && kb + 4 < ZP) { eyk = __ldg(P.e[1] + g + 4); exk = __ldg(P.e[0] + g + 4); }
-        ldg4v(P.h[0] + g, hx); ldg4v(P.h[1] + g, hy); ldg4v(P.h[2] + g, hz);
-        if (by) ld4v(P.pi[0] + g, p0);
-        if (vyH && bz) ld4v(P.pi[1] + g, p1);
-        if (xok && bz) ld4v(P.pi[2] + g, p2);
-        if (bx) ld4v(P.pi[3] + g, p3);
-        if (vyH && bx) ld4v(P.pi[4] + g, p4);
-        if (xok && by) ld4v(P.pi[5] + g, p5);
+        ldg4v(P.e[FA] + g, fa);
+        ldg4v(P.e[FB] + g, fb);
+        if (AA == 1 && j + 1 < ny) ldg4v(P.e[FA] + g + ZP, fan);
+        if (AA == 0 && i + 1 < nx) ldg4v(P.e[FA] + g + NYZ, fan);
+        if (AB == 1 && j + 1 < ny) ldg4v(P.e[FB] + g + ZP, fbn);
+        if (AB == 0 && i + 1 < nx) ldg4v(P.e[FB] + g + NYZ, fbn);
+        if (C != 2 && (threadIdx.x & 31) == 31 && kb + 4 < ZP)
+            zk = __ldg(P.e[AA == 2 ? FA : FB] + g + 4);
+        ldg4v(P.h[C] + g, h);
+        if (pa_on) ldg4v(P.pi[2 * C] + g, pa);
+        if (pb_on) ldg4v(P.pi[2 * C + 1] + g, pb);
     }
-    // profiles (tiny, cache resident); (1, 0) outside the bands
-    float hxb = 1.f, hxa = 0.f, hyb = 1.f, hya = 0.f, hzb[4], hza[4];
-    if (bx) { hxb = __ldg(P.pb[0][0] + i); hxa = __ldg(P.pa[0][0] + i); }
-    if (by) { hyb = __ldg(P.pb[1][0] + j); hya = __ldg(P.pa[1][0] + j); }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const bool on = bz && kb + q <= nz - 2;
-        hzb[q] = on ? __ldg(P.pb[2][0] + kb + q) : 1.f;
-        hza[q] = on ? __ldg(P.pa[2][0] + kb + q) : 0.f;
+    float a1[4], a2[4];
+    if (DAMP && act) {
+        ldg4v(P.dmp[3 + C][0] + g, a1);
+        ldg4v(P.dmp[3 + C][1] + g, a2);
     }
-    {
-        const float t0 = __shfl_down_sync(0xffffffffu, ey[0], 1);   // E(k+1) of q = 3
-        const float t1 = __shfl_down_sync(0xffffffffu, ex[0], 1);
-        if (lane != 31) { eyk = t0; exk = t1; }
+    // profile of the x or y term; (1, 0) outside the bands (tiny, cache resident)
+    float b0 = 1.f, a0 = 0.f, b1 = 1.f, a1p = 0.f;        // first x / y term; second (Hz: y)
+    if (C == 0 && by) { b0 = __ldg(P.pb[1][0] + j); a0 = __ldg(P.pa[1][0] + j); }
+    if (C != 0 && bx) { b0 = __ldg(P.pb[0][0] + i); a0 = __ldg(P.pa[0][0] + i); }
+    if (C == 2 && by) { b1 = __ldg(P.pb[1][0] + j); a1p = __ldg(P.pa[1][0] + j); }
+    if (C != 2) {
+        const float t = __shfl_down_sync(0xffffffffu, AA == 2 ? fa[0] : fb[0], 1);
+        if ((threadIdx.x & 31) != 31) zk = t;
+        float(&f)[4] = AA == 2 ? fa : fb;
+        float(&fn)[4] = AA == 2 ? fan : fbn;
+        fn[0] = f[1]; fn[1] = f[2]; fn[2] = f[3]; fn[3] = zk;
     }
     if (!act) return;
-    float a1[3][4], a2[3][4];
-    if (DAMP) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            ldg4v(P.dmp[3 + c][0] + g, a1[c]);
-            ldg4v(P.dmp[3 + c][1] + g, a2[c]);
-        }
-    }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const bool vz = kb + q <= nz - 2, vzE = kb + q < nz;
-        const float eyn = (q < 3) ? ey[q + 1] : eyk;
-        const float exn = (q < 3) ? ex[q + 1] : exk;
-        // Hx: valid j <= ny-2, k <= nz-2
-        {
-            float qy, qz;
-            const float cu = __fsub_rn(y3_s(y3_d(ezj[q], ez[q], rdx), hyb, hya, p0[q], qy),
-                                       y3_s(y3_d(eyn, ey[q], rdx), hzb[q], hza[q], p1[q], qz));
-            const bool v = vyH && vz;
-            const float hn = DAMP ? y3_hd(hx[q], cu, a1[0][q], a2[0][q]) : y3_h(hx[q], cu, dt);
-            hx[q] = v ? hn : hx[q];
-            p0[q] = v ? qy : p0[q];
-            p1[q] = v ? qz : p1[q];
-        }
-        // Hy: valid i <= nx-2, k <= nz-2
-        {
-            float qz, qx;
-            const float cu = __fsub_rn(y3_s(y3_d(exn, ex[q], rdx), hzb[q], hza[q], p2[q], qz),
-                                       y3_s(y3_d(ezi[q], ez[q], rdx), hxb, hxa, p3[q], qx));
-            const bool v = xok && vz;
-            const float hn = DAMP ? y3_hd(hy[q], cu, a1[1][q], a2[1][q]) : y3_h(hy[q], cu, dt);
-            hy[q] = v ? hn : hy[q];
-            p2[q] = v ? qz : p2[q];
-            p3[q] = v ? qx : p3[q];
-        }
-        // Hz: valid i <= nx-2, j <= ny-2, k < nz
-        {
-            float qx, qy;
-            const float cu = __fsub_rn(y3_s(y3_d(eyi[q], ey[q], rdx), hxb, hxa, p4[q], qx),
-                                       y3_s(y3_d(exj[q], ex[q], rdx), hyb, hya, p5[q], qy));
-            const bool v = xok && vyH && vzE;
-            const float hn = DAMP ? y3_hd(hz[q], cu, a1[2][q], a2[2][q]) : y3_h(hz[q], cu, dt);
-            hz[q] = v ? hn : hz[q];
-            p4[q] = v ? qx : p4[q];
-            p5[q] = v ? qy : p5[q];
-        }
+        const int k = kb + q;
+        const bool vz = k <= nz - 2, vzE = k < nz;
+        const bool v = C == 0 ? (vyH && vz) : C == 1 ? (xok && vz) : (xok && vyH && vzE);
+        float zb = 1.f, za = 0.f;
+        if (C != 2) s3_zprof(P.pb[2][0], P.pa[2][0], bz && vz, k, zb, za);
+        const float ta = s3_term(fan[q], fa[q], rdx, AA == 2 ? zb : b0, AA == 2 ? za : a0, pa[q], v);
+        const float tb = s3_term(fbn[q], fb[q], rdx, AB == 2 ? zb : C == 2 ? b1 : b0,
+                                 AB == 2 ? za : C == 2 ? a1p : a0, pb[q], v);
+        const float cu = __fsub_rn(ta, tb);
+        const float hn = DAMP ? y3_hd(h[q], cu, a1[q], a2[q]) : y3_h(h[q], cu, P.dt);
+        h[q] = v ? hn : h[q];
     }
-    st4v(P.ho[0] + g, hx);
-    st4v(P.ho[1] + g, hy);
-    st4v(P.ho[2] + g, hz);
-    if (by) st4v(P.po[0] + g, p0);
-    if (vyH && bz) st4v(P.po[1] + g, p1);
-    if (xok && bz) st4v(P.po[2] + g, p2);
-    if (bx) st4v(P.po[3] + g, p3);
-    if (vyH && bx) st4v(P.po[4] + g, p4);
-    if (xok && by) st4v(P.po[5] + g, p5);
+    st4v(P.ho[C] + g, h);
+    if (pa_on) st4v(P.po[2 * C] + g, pa);
+    if (pb_on) st4v(P.po[2 * C + 1] + g, pb);
 }
 
-// E(n+1) from H(n+1/2) and E(n): core/stepper_3d.py:395-437, source
+template <bool DAMP>
+__global__ void __launch_bounds__(3 * S3_T, 3) k_yee3d_h(const __grid_constant__ Split3 P, int i0) {
+    const S3Cell c(P, i0 + blockIdx.y);
+    if (threadIdx.y == 0) s3_h<0, DAMP>(P, c);
+    else if (threadIdx.y == 1) s3_h<1, DAMP>(P, c);
+    else s3_h<2, DAMP>(P, c);
+}
+
+// E(n+1) of component C from H(n+1/2) and E(n): core/stepper_3d.py:395-437, source
 // :448-482. The E-side psi recursions run over their arrays' full extent
 // (core/stepper_3d.py:79-101 State3D shapes), wider than the interior where
 // the curl is applied (_pad_interior). E(n+1) = E(n) + dt curl / eps_c with a
 // fast (2 ulp) divide; the reference's (E eps + dt curl) / eps differs by
-// rounding only.
-template <int MODE>                 // bit 0: damping, bit 1: poles
-__global__ void __launch_bounds__(32 * SPLIT_Y, 2) k_yee3d_e(const __grid_constant__ Split3 P,
-                                                             const float *__restrict__ amp, int i0) {
+// rounding only. MODE bit 0: damping, bit 1: poles.
+template <int C, int MODE>
+__device__ __forceinline__ void s3_e(const Split3 &P, const S3Cell &c,
+                                     const float *__restrict__ amp) {
     constexpr bool DAMP = (MODE & 1) != 0, PL = (MODE & 2) != 0;
     const int nx = P.nx, ny = P.ny, nz = P.nz, ZP = P.zp;
-    const int lane = threadIdx.x;
-    const int j = blockIdx.y * SPLIT_Y + threadIdx.y;
-    const int i = i0 + blockIdx.z;
-    const int kb = blockIdx.x * 128 + 4 * lane;
-    const bool act = j < ny && kb < ZP;
-    const uint32_t NYZ = (uint32_t)ny * ZP;       // box < 2^31 elements (plan check)
-    const uint32_t g = (uint32_t)i * NYZ + (uint32_t)(j * ZP + kb);
-    const float dt = P.dt, rdx = P.rdx;
+    const int i = c.i, j = c.j, kb = c.kb;
+    const uint32_t g = c.g, NYZ = (uint32_t)ny * ZP;
+    const float rdx = P.rdx;
+    const int lane = threadIdx.x & 31;
+    const bool act = c.act;
     const bool iin = i >= 1 && i <= nx - 2, jin = j >= 1 && j <= ny - 2;
     const bool pmx = P.pmc & 1, pmy = (P.pmc >> 1) & 1, pmz = (P.pmc >> 2) & 1;
     const bool xok = i <= nx - 2, vyH = j <= ny - 2;
@@ -659,181 +665,140 @@ __global__ void __launch_bounds__(32 * SPLIT_Y, 2) k_yee3d_e(const __grid_consta
         const int k = kb + q;
         bz |= k >= 1 && k <= nz - 2 && inband(P.B, 2, 1, k);
     }
-    const float *__restrict__ Hx = P.ho[0];
-    const float *__restrict__ Hy = P.ho[1];
-    const float *__restrict__ Hz = P.ho[2];
-    const float *__restrict__ eps = P.eps;
-    float hx[4], hy[4], hz[4], ep[4], hzm[4], hxm[4], hzp[4], hyp[4], epj[4], epi[4], en[3][4];
-    float p6[4], p7[4], p8[4], p9[4], p10[4], p11[4];
-    float hyk = 0.f, hxk = 0.f, epk = 1.f;
-    z4(hx); z4(hy); z4(hz); one4(ep); z4(hzm); z4(hxm); z4(hzp); z4(hyp); one4(epj); one4(epi);
-    z4(p6); z4(p7); z4(p8); z4(p9); z4(p10); z4(p11);
-    z4(en[0]); z4(en[1]); z4(en[2]);
-    int e0 = 0, e1x = 0;                          // soft current cells of row (i, j)
+    // Ex: dy Hz (psi 6), dz Hy (psi 7); Ey: dz Hx (psi 8), dx Hz (psi 9);
+    // Ez: dx Hy (psi 10), dy Hx (psi 11)
+    constexpr int FA = C == 0 ? 2 : C == 1 ? 0 : 1;      // first term's H component
+    constexpr int FB = C == 0 ? 1 : C == 1 ? 2 : 0;
+    constexpr int AA = C == 0 ? 1 : C == 1 ? 2 : 0;      // its axis (0 x, 1 y, 2 z)
+    constexpr int AB = C == 0 ? 2 : C == 1 ? 0 : 1;
+    const bool pa_on = C == 0 ? (xok && by) : C == 1 ? (vyH && bz) : bx;
+    const bool pb_on = C == 0 ? (xok && bz) : C == 1 ? (vyH && bx) : by;
+    const float *__restrict__ Ha = P.ho[FA];
+    const float *__restrict__ Hb = P.ho[FB];
+    float ha[4], hap[4], hb[4], hbp[4], ep[4], epn[4], en[4], pa[4], pb[4];
+    z4(ha); z4(hap); z4(hb); z4(hbp); one4(ep); one4(epn); z4(en); z4(pa); z4(pb);
+    float zk = 0.f, epk = 1.f;                            // H(k-1) of q = 0, eps(k+1) of q = 3
+    int e0 = 0, e1x = 0;                                  // soft current cells of row (i, j)
+    float pc[4], pq[4], c3[4];                            // first pole: P(n), P(n-1), drive
     if (act) {
-        ldg4v(Hx + g, hx); ldg4v(Hy + g, hy); ldg4v(Hz + g, hz); ldg4v(eps + g, ep);
-        if (j >= 1) { ldg4v(Hz + g - ZP, hzm); ldg4v(Hx + g - ZP, hxm); }
-        if (i >= 1) { ldg4v(Hz + g - NYZ, hzp); ldg4v(Hy + g - NYZ, hyp); }
-        if (j + 1 < ny) ldg4v(eps + g + ZP, epj);
-        if (i + 1 < nx) ldg4v(eps + g + NYZ, epi);
-        if (lane == 0 && kb >= 1) { hyk = __ldg(Hy + g - 1); hxk = __ldg(Hx + g - 1); }
-        if (lane == 31 && kb + 4 < ZP) epk = __ldg(eps + g + 4);
-        ldg4v(P.e[0] + g, en[0]); ldg4v(P.e[1] + g, en[1]); ldg4v(P.e[2] + g, en[2]);
-        if (xok && by) ld4v(P.pi[6] + g, p6);
-        if (xok && bz) ld4v(P.pi[7] + g, p7);
-        if (vyH && bz) ld4v(P.pi[8] + g, p8);
-        if (vyH && bx) ld4v(P.pi[9] + g, p9);
-        if (bx) ld4v(P.pi[10] + g, p10);
-        if (by) ld4v(P.pi[11] + g, p11);
-        if (P.src_n > 0) {
+        ldg4v(Ha + g, ha);
+        ldg4v(Hb + g, hb);
+        ldg4v(P.eps + g, ep);
+        ldg4v(P.e[C] + g, en);
+        if (AA == 1 && j >= 1) ldg4v(Ha + g - ZP, hap);
+        if (AA == 0 && i >= 1) ldg4v(Ha + g - NYZ, hap);
+        if (AB == 1 && j >= 1) ldg4v(Hb + g - ZP, hbp);
+        if (AB == 0 && i >= 1) ldg4v(Hb + g - NYZ, hbp);
+        if (C == 0 && i + 1 < nx) ldg4v(P.eps + g + NYZ, epn);
+        if (C == 1 && j + 1 < ny) ldg4v(P.eps + g + ZP, epn);
+        if (C == 2 && lane == 31 && kb + 4 < ZP) epk = __ldg(P.eps + g + 4);
+        if (C != 2 && lane == 0 && kb >= 1) zk = __ldg((AA == 2 ? Ha : Hb) + g - 1);
+        if (pa_on) ldg4v(P.pi[6 + 2 * C] + g, pa);
+        if (pb_on) ldg4v(P.pi[7 + 2 * C] + g, pb);
+        if (PL) {
+            ld4v(P.pp[C][0] + g, pc);
+            ld4v(P.pp[C][1] + g, pq);
+            ldg4v(P.pc3[C] + g, c3);
+        }
+        if (P.src_n > 0 && P.src_comp == C) {
             e0 = __ldg(P.src_row + i * ny + j);
             e1x = __ldg(P.src_row + i * ny + j + 1);
         }
     }
-    float exb = 1.f, exa = 0.f, eyb = 1.f, eya = 0.f, ezb[4], eza[4];
-    if (bx) { exb = __ldg(P.pb[0][1] + i); exa = __ldg(P.pa[0][1] + i); }
-    if (by) { eyb = __ldg(P.pb[1][1] + j); eya = __ldg(P.pa[1][1] + j); }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int k = kb + q;
-        const bool on = bz && k >= 1 && k <= nz - 2;
-        ezb[q] = on ? __ldg(P.pb[2][1] + k) : 1.f;
-        eza[q] = on ? __ldg(P.pa[2][1] + k) : 0.f;
+    // conductive damping: E' = d1 E + d2 curl / eps (core/stepper_3d.py:405-437)
+    float a1[4], a2[4];
+    if (DAMP && act) {
+        ldg4v(P.dmp[C][0] + g, a1);
+        ldg4v(P.dmp[C][1] + g, a2);
     }
-    {
-        const float t0 = __shfl_up_sync(0xffffffffu, hy[3], 1);     // H(k-1) of q = 0
-        const float t1 = __shfl_up_sync(0xffffffffu, hx[3], 1);
-        const float t2 = __shfl_down_sync(0xffffffffu, ep[0], 1);   // eps(k+1) of q = 3
-        if (lane != 0) { hyk = t0; hxk = t1; }
-        if (lane != 31) epk = t2;
+    float b0 = 1.f, a0 = 0.f, b1 = 1.f, a1p = 0.f;        // x / y profile; Ez's y term
+    if (C == 0 && by) { b0 = __ldg(P.pb[1][1] + j); a0 = __ldg(P.pa[1][1] + j); }
+    if (C != 0 && bx) { b0 = __ldg(P.pb[0][1] + i); a0 = __ldg(P.pa[0][1] + i); }
+    if (C == 2 && by) { b1 = __ldg(P.pb[1][1] + j); a1p = __ldg(P.pa[1][1] + j); }
+    if (C != 2) {
+        const float t = __shfl_up_sync(0xffffffffu, AA == 2 ? ha[3] : hb[3], 1);
+        if (lane != 0) zk = t;
+        if (kb == 0) zk = 0.f;                            // the lane before is another row
+        float(&f)[4] = AA == 2 ? ha : hb;
+        float(&fp)[4] = AA == 2 ? hap : hbp;
+        fp[0] = zk; fp[1] = f[0]; fp[2] = f[1]; fp[3] = f[2];
+    } else {
+        const float t = __shfl_down_sync(0xffffffffu, ep[0], 1);
+        if (lane != 31) epk = t;
+        if (kb + 4 >= ZP) epk = 1.f;
+        epn[0] = ep[1]; epn[1] = ep[2]; epn[2] = ep[3]; epn[3] = epk;
     }
     if (!act) return;
-    // conductive damping: E' = d1 E + d2 curl / eps (core/stepper_3d.py:405-437)
-    float a1[3][4], a2[3][4];
-    if (DAMP) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            ldg4v(P.dmp[c][0] + g, a1[c]);
-            ldg4v(P.dmp[c][1] + g, a2[c]);
-        }
-    }
     // dispersive poles (core/stepper_3d.py:295-300, :312-325): P(n+1) = c1 P(n) +
     // c2 P(n-1) + c3 E(n) over the P(n-1) buffer, and the sums of P(n), P(n+1) that the
     // folded-D update E(n+1) = (d1 (eps E + sum P(n)) + d2 curl - sum P(n+1)) / eps needs
-    float spc[3][4], spn[3][4];
+    float spc[4], spn[4];
     if (PL) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            z4(spc[c]);
-            z4(spn[c]);
+        z4(spc);
+        z4(spn);
 #pragma unroll 1
-            for (int k = 0; k < P.np; ++k) {
-                const uint32_t o = k * P.plane + g;
-                float pc[4], pq[4], c3[4];
-                ld4v(P.pp[c][0] + o, pc);
-                ld4v(P.pp[c][1] + o, pq);
-                ldg4v(P.pc3[c] + o, c3);
-                const float c1 = P.pc1[k], c2 = P.pc2[k];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    spc[c][q] += pc[q];
-                    pq[q] = __fmaf_rn(c3[q], en[c][q], __fmaf_rn(c2, pq[q], __fmul_rn(c1, pc[q])));
-                    spn[c][q] += pq[q];
-                }
-                st4v(P.pp[c][1] + o, pq);
+        for (int k = 0; k < P.np; ++k) {
+            const uint32_t o = k * P.plane + g;
+            if (k > 0) {
+                ld4v(P.pp[C][0] + o, pc);
+                ld4v(P.pp[C][1] + o, pq);
+                ldg4v(P.pc3[C] + o, c3);
             }
+            const float c1 = P.pc1[k], c2 = P.pc2[k];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                spc[q] += pc[q];
+                pq[q] = __fmaf_rn(c3[q], en[q], __fmaf_rn(c2, pq[q], __fmul_rn(c1, pc[q])));
+                spn[q] += pq[q];
+            }
+            st4v(P.pp[C][1] + o, pq);
         }
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int k = kb + q;
         const bool vzE = k < nz, vz = k <= nz - 2, kin = k >= 1 && k <= nz - 2;
-        const float hym = (q == 0) ? hyk : hy[q - 1];
-        const float hxkm = (q == 0) ? hxk : hx[q - 1];
-        // Ex: valid i <= nx-2, k < nz; curl on j, k interior
-        {
-            float qy, qz;
-            const float ty = y3_s(y3_d(hz[q], hzm[q], rdx), eyb, eya, p6[q], qy);
-            const float tz = y3_s(y3_d(hy[q], hym, rdx), ezb[q], eza[q], p7[q], qz);
-            const bool v = xok && vzE;
-            const float curl = y3_curl(ty, !jin, pmy, tz, !kin, pmz);
-            const float ec = y3_ec(ep[q], epi[q]);
-            en[0][q] = v ? (PL ? (DAMP ? y3_epd(en[0][q], curl, a1[0][q], a2[0][q], ec, spc[0][q],
-                                                spn[0][q])
-                                       : y3_ep(en[0][q], curl, dt, ec, spc[0][q], spn[0][q]))
-                                 : DAMP ? y3_ed(en[0][q], curl, a1[0][q], a2[0][q], ec)
-                                        : y3_e(en[0][q], curl, dt, ec))
-                         : en[0][q];
-            p6[q] = v ? qy : p6[q];
-            p7[q] = v ? qz : p7[q];
-        }
-        // Ey: valid j <= ny-2, k < nz; curl on i, k interior
-        {
-            float qz, qx;
-            const float tz = y3_s(y3_d(hx[q], hxkm, rdx), ezb[q], eza[q], p8[q], qz);
-            const float tx = y3_s(y3_d(hz[q], hzp[q], rdx), exb, exa, p9[q], qx);
-            const bool v = vyH && vzE;
-            const float curl = y3_curl(tz, !kin, pmz, tx, !iin, pmx);
-            const float ec = y3_ec(ep[q], epj[q]);
-            en[1][q] = v ? (PL ? (DAMP ? y3_epd(en[1][q], curl, a1[1][q], a2[1][q], ec, spc[1][q],
-                                                spn[1][q])
-                                       : y3_ep(en[1][q], curl, dt, ec, spc[1][q], spn[1][q]))
-                                 : DAMP ? y3_ed(en[1][q], curl, a1[1][q], a2[1][q], ec)
-                                        : y3_e(en[1][q], curl, dt, ec))
-                         : en[1][q];
-            p8[q] = v ? qz : p8[q];
-            p9[q] = v ? qx : p9[q];
-        }
-        // Ez: valid k <= nz-2; curl on i, j interior
-        {
-            float qx, qy;
-            const float tx = y3_s(y3_d(hy[q], hyp[q], rdx), exb, exa, p10[q], qx);
-            const float ty = y3_s(y3_d(hx[q], hxm[q], rdx), eyb, eya, p11[q], qy);
-            const float curl = y3_curl(tx, !iin, pmx, ty, !jin, pmy);
-            const float ec = y3_ec(ep[q], (q < 3) ? ep[q + 1] : epk);
-            en[2][q] = vz ? (PL ? (DAMP ? y3_epd(en[2][q], curl, a1[2][q], a2[2][q], ec, spc[2][q],
-                                                 spn[2][q])
-                                        : y3_ep(en[2][q], curl, dt, ec, spc[2][q], spn[2][q]))
-                                  : DAMP ? y3_ed(en[2][q], curl, a1[2][q], a2[2][q], ec)
-                                         : y3_e(en[2][q], curl, dt, ec))
-                          : en[2][q];
-            p10[q] = vz ? qx : p10[q];
-            p11[q] = vz ? qy : p11[q];
-        }
+        const bool v = C == 0 ? (xok && vzE) : C == 1 ? (vyH && vzE) : vz;
+        float zb = 1.f, za = 0.f;
+        if (C != 2) s3_zprof(P.pb[2][1], P.pa[2][1], bz && kin, k, zb, za);
+        const float ta = s3_term(ha[q], hap[q], rdx, AA == 2 ? zb : b0, AA == 2 ? za : a0, pa[q], v);
+        const float tb = s3_term(hb[q], hbp[q], rdx, AB == 2 ? zb : C == 2 ? b1 : b0,
+                                 AB == 2 ? za : C == 2 ? a1p : a0, pb[q], v);
+        const float curl = C == 0 ? y3_curl(ta, !jin, pmy, tb, !kin, pmz)
+                         : C == 1 ? y3_curl(ta, !kin, pmz, tb, !iin, pmx)
+                                  : y3_curl(ta, !iin, pmx, tb, !jin, pmy);
+        const float ec = y3_ec(ep[q], epn[q]);
+        const float e1 = PL ? (DAMP ? y3_epd(en[q], curl, a1[q], a2[q], ec, spc[q], spn[q])
+                                    : y3_ep(en[q], curl, P.dt, ec, spc[q], spn[q]))
+                            : DAMP ? y3_ed(en[q], curl, a1[q], a2[q], ec)
+                                   : y3_e(en[q], curl, P.dt, ec);
+        en[q] = v ? e1 : en[q];
     }
     // soft current cells of row (i, j) on component src_comp
     if (e0 < e1x) {
-        const int c = P.src_comp;
         const float a = __ldg(amp);
         const float sgn = P.src_is_point ? (float)P.point_sign : -1.f;
         for (int e = e0; e < e1x; ++e) {
             const int kq = __ldg(P.src_col + e) - kb;
+            const float v = __fmul_rn(a, __ldg(P.src_w + e));
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                if (kq != q) continue;
-                float epn;
-                if (c == 0) epn = epi[q];
-                else if (c == 1) epn = epj[q];
-                else epn = (q < 3) ? ep[q + 1] : epk;
-                const float ecomp = y3_ec(ep[q], epn);
-                const float v = __fmul_rn(a, __ldg(P.src_w + e));
-#pragma unroll
-                for (int cc = 0; cc < 3; ++cc) {         // static component index
-                    if (cc != c) continue;
-                    en[cc][q] = y3_src(en[cc][q], v, ecomp, P.src_is_point != 0, sgn);
-                }
-            }
+            for (int q = 0; q < 4; ++q)
+                if (kq == q)
+                    en[q] = y3_src(en[q], v, y3_ec(ep[q], epn[q]), P.src_is_point != 0, sgn);
         }
     }
-    st4v(P.eo[0] + g, en[0]);
-    st4v(P.eo[1] + g, en[1]);
-    st4v(P.eo[2] + g, en[2]);
-    if (xok && by) st4v(P.po[6] + g, p6);
-    if (xok && bz) st4v(P.po[7] + g, p7);
-    if (vyH && bz) st4v(P.po[8] + g, p8);
-    if (vyH && bx) st4v(P.po[9] + g, p9);
-    if (bx) st4v(P.po[10] + g, p10);
-    if (by) st4v(P.po[11] + g, p11);
+    st4v(P.eo[C] + g, en);
+    if (pa_on) st4v(P.po[6 + 2 * C] + g, pa);
+    if (pb_on) st4v(P.po[7 + 2 * C] + g, pb);
+}
+
+template <int MODE>                 // bit 0: damping, bit 1: poles
+__global__ void __launch_bounds__(3 * S3_T, MODE ? 2 : 3)
+k_yee3d_e(const __grid_constant__ Split3 P, const float *__restrict__ amp, int i0) {
+    const S3Cell c(P, i0 + blockIdx.y);
+    if (threadIdx.y == 0) s3_e<0, MODE>(P, c, amp);
+    else if (threadIdx.y == 1) s3_e<1, MODE>(P, c, amp);
+    else s3_e<2, MODE>(P, c, amp);
 }
 
 // Copy the plane samples of the (new) state into one ring slot.
@@ -1200,14 +1165,24 @@ int mtb_yee3d_plan_create(const mtb_yee3d_struct *s, const mtb_dft_region *regio
     const bool xm_ok = n_damp0 == 0 && S.n_poles == 0 && S.zpitch <= 256;
     if (asked == 3 && !xm_ok)
         return fail(MTB_UNSUPPORTED, "one-pass 3D kernel: no damping or poles, zpitch <= 256");
-    const int variant = asked == 1 ? 1 : (asked == 3 || (asked == 0 && xm_ok)) ? 3 : 2;
+    // The one-pass kernel marches each block through planes one after the other, 3 us a
+    // plane, and wants enough planes per block and full 128-wide rows to be worth it.
+    // Measured, split / one-pass us per step: 117 x 90 x 75 24 / 37, 128^3 52 / 54,
+    // 192^3 149 / 161 (rows 3/4 full), 256 x 256 x 128 175 / 171, 224^3 227 / 213, 256^3
+    // 331 / 282; 400 x 400 x 64 217 / 353 (half-full rows). So: 8 M cells or more and
+    // rows filled to at least 4/5.
+    const int xm_row = S.zpitch <= 128 ? 128 : 256;
+    const bool xm_pays = (int64_t)S.nx * S.ny * S.nz >= (8 << 20) &&
+                         (int64_t)S.zpitch * 5 >= 4 * xm_row;
+    const int variant = asked == 1 ? 1
+                                   : (asked == 3 || (asked == 0 && xm_ok && xm_pays)) ? 3 : 2;
     if (variant == 1 && S.zpitch > 128 * MAXNZ)
         return fail(MTB_UNSUPPORTED, "fused kernel: zpitch %d > %d not supported", S.zpitch,
                     128 * MAXNZ);
-    if (variant != 1 && (S.nx > 65535 || (S.ny + SPLIT_Y - 1) / SPLIT_Y > 65535 ||
+    if (variant != 1 && (S.nx > 65535 || S.ny > 65535 * 8 ||
                          (int64_t)S.nx * S.ny * S.zpitch >= (1LL << 31)))
         return fail(MTB_UNSUPPORTED, "split kernels: nx <= 65535, ny <= %d, box < 2^31 cells",
-                    65535 * SPLIT_Y);
+                    65535 * 8);
     if ((int64_t)S.nx * S.ny * S.zpitch >= (1LL << 34))
         return fail(MTB_UNSUPPORTED, "grid too large");
     if ((int64_t)S.nx * S.ny >= (1LL << 31)) return fail(MTB_UNSUPPORTED, "nx*ny too large");
@@ -1417,22 +1392,23 @@ static int stage_chunk(mtb_yee3d_plan *p, int64_t t0, int k, const double *coef,
 
 // Split-kernel H (part 0) or E (part 1) update of x planes [i0, i1), step s
 // of the staged chunk.
-static int launch_split(mtb_yee3d_plan *p, int part, int i0, int i1, int s, cudaStream_t st) {
+static int launch_split(mtb_yee3d_plan *p, const Split3 &sp, int part, int i0, int i1, int s,
+                        cudaStream_t st) {
     if (i1 <= i0) return MTB_OK;
-    const dim3 grid((p->s.zpitch + 127) / 128, (p->s.ny + SPLIT_Y - 1) / SPLIT_Y, i1 - i0);
-    const dim3 block(32, SPLIT_Y);
+    const dim3 grid((unsigned)(((int64_t)p->s.ny * (p->s.zpitch / 4) + S3_T - 1) / S3_T), i1 - i0);
+    const dim3 block(S3_T, 3);
     if (part == 0) {
         if (p->damp)
-            k_yee3d_h<true><<<grid, block, 0, st>>>(p->sp[p->par], i0);
+            k_yee3d_h<true><<<grid, block, 0, st>>>(sp, i0);
         else
-            k_yee3d_h<false><<<grid, block, 0, st>>>(p->sp[p->par], i0);
+            k_yee3d_h<false><<<grid, block, 0, st>>>(sp, i0);
     } else {
         const float *a = p->amp_d.as<float>() + s;
         switch ((p->damp ? 1 : 0) | (p->poles ? 2 : 0)) {
-            case 0: k_yee3d_e<0><<<grid, block, 0, st>>>(p->sp[p->par], a, i0); break;
-            case 1: k_yee3d_e<1><<<grid, block, 0, st>>>(p->sp[p->par], a, i0); break;
-            case 2: k_yee3d_e<2><<<grid, block, 0, st>>>(p->sp[p->par], a, i0); break;
-            default: k_yee3d_e<3><<<grid, block, 0, st>>>(p->sp[p->par], a, i0); break;
+            case 0: k_yee3d_e<0><<<grid, block, 0, st>>>(sp, a, i0); break;
+            case 1: k_yee3d_e<1><<<grid, block, 0, st>>>(sp, a, i0); break;
+            case 2: k_yee3d_e<2><<<grid, block, 0, st>>>(sp, a, i0); break;
+            default: k_yee3d_e<3><<<grid, block, 0, st>>>(sp, a, i0); break;
         }
     }
     MTB_CHECK_LAUNCH();
@@ -1502,8 +1478,8 @@ int mtb_yee3d_run(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, 
             const int ns = p->slab;
             for (int i0 = p->own_lo; i0 < p->own_hi; i0 += ns) {
                 const int i1 = std::min(i0 + ns, p->own_hi);
-                if ((rc = launch_split(p, 0, i0, i1, s, st))) return rc;
-                if ((rc = launch_split(p, 1, i0, i1, s, st))) return rc;
+                if ((rc = launch_split(p, p->sp[p->par], 0, i0, i1, s, st))) return rc;
+                if ((rc = launch_split(p, p->sp[p->par], 1, i0, i1, s, st))) return rc;
             }
         }
         if ((rc = p->timer.end(st))) return rc;
@@ -1560,13 +1536,50 @@ int mtb_yee3d_half(mtb_yee3d_plan *p, int32_t part, void *stream) {
     int rc;
     if (part == 0) {
         if ((rc = p->timer.begin(st, 0))) return rc;
-        if ((rc = launch_split(p, 0, p->own_lo, p->own_hi, p->c_s, st))) return rc;
+        if ((rc = launch_split(p, p->sp[p->par], 0, p->own_lo, p->own_hi, p->c_s, st))) return rc;
         p->c_half = 1;
         return MTB_OK;
     }
-    if ((rc = launch_split(p, 1, p->own_lo, p->own_hi, p->c_s, st))) return rc;
+    if ((rc = launch_split(p, p->sp[p->par], 1, p->own_lo, p->own_hi, p->c_s, st))) return rc;
     if ((rc = p->timer.end(st))) return rc;
     return finish_step(p, st);
+}
+
+int mtb_yee3d_run_record(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, float *rec,
+                         int64_t rec_comp_stride, int64_t rec_slot_stride, void *stream) {
+    if (!p) return fail(MTB_INVALID_ARG, "plan is null");
+    if (int rc = need_split(p, "recorded steps")) return rc;
+    if (k < 0) return fail(MTB_INVALID_ARG, "k < 0");
+    if (!rec || (reinterpret_cast<uintptr_t>(rec) & 15) || (rec_comp_stride & 3) ||
+        (rec_slot_stride & 3))
+        return fail(MTB_INVALID_ARG, "record: null or unaligned");
+    if (p->own_lo != 0 || p->own_hi != p->s.nx)
+        return fail(MTB_UNSUPPORTED, "recorded steps of an x slab");
+    p->last_launches = 0;
+    if (k == 0) return MTB_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc;
+    if ((rc = stage_chunk(p, t0, k, coef, st))) return rc;
+    const size_t bytes = sizeof(float) * (size_t)p->s.nx * p->s.ny * p->s.zpitch;
+    for (int c = 0; c < 3; ++c)
+        MTB_CUDA_TRY(cudaMemcpyAsync(rec + c * rec_comp_stride, p->s.f[c][p->par], bytes,
+                                     cudaMemcpyDeviceToDevice, st));
+    for (int s = 0; s < k; ++s) {
+        Split3 sp = p->sp[p->par];
+        for (int c = 0; c < 3; ++c) {
+            sp.e[c] = rec + (size_t)s * rec_slot_stride + c * rec_comp_stride;
+            sp.eo[c] = rec + (size_t)(s + 1) * rec_slot_stride + c * rec_comp_stride;
+        }
+        if ((rc = launch_split(p, sp, 0, 0, p->s.nx, s, st))) return rc;
+        if ((rc = launch_split(p, sp, 1, 0, p->s.nx, s, st))) return rc;
+        p->par ^= 1;
+    }
+    p->c_s = p->c_k;                       // no staged step left
+    for (int c = 0; c < 3; ++c)            // the live E buffers hold the last step's E
+        MTB_CUDA_TRY(cudaMemcpyAsync(p->s.f[c][p->par],
+                                     rec + (size_t)k * rec_slot_stride + c * rec_comp_stride,
+                                     bytes, cudaMemcpyDeviceToDevice, st));
+    return MTB_OK;
 }
 
 int mtb_yee3d_set_timing(mtb_yee3d_plan *p, int32_t enable) {

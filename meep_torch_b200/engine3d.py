@@ -392,6 +392,21 @@ class Engine3D:
         L.check(self.lib.mtb_yee3d_run(self.plan, t0, k, coef, self._sptr()), "mtb_yee3d_run")
         self.last_launches = self.lib.mtb_yee3d_last_launches(self.plan)
 
+    def run_record(self, t0: int, k: int, record: torch.Tensor):
+        """Advance k steps on the split kernels without monitor samples, keeping E before
+        and after every step in ``record`` (at least k + 1, 3, nx, ny, zpitch)."""
+        coef = None
+        if self.source is not None:
+            v = coef_table(self.source, "amplitude", t0, k, self._dt)
+            self._coef = np.ascontiguousarray(v, dtype=np.float64)
+            coef = self._coef.ctypes.data_as(C.POINTER(C.c_double))
+        n = self.nx * self.ny * self.zp
+        _need(record.is_contiguous() and record.numel() >= (k + 1) * 3 * n,
+              "run_record: record of at least (k + 1, 3, nx, ny, zpitch)")
+        L.check(self.lib.mtb_yee3d_run_record(self.plan, t0, k, coef, L.ptr(record), n, 3 * n,
+                                              self._sptr()), "mtb_yee3d_run_record")
+        self.last_launches = self.lib.mtb_yee3d_last_launches(self.plan)
+
     def begin(self, t0: int, k: int):
         """Stage steps t0 .. t0+k-1 for half(); the amplitudes as in run()."""
         coef = None
