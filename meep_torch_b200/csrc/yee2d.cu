@@ -2063,6 +2063,7 @@ namespace mtb {
 
 #include "yee2d_tb.cuh"
 #include "yee2d_cl.cuh"
+#include "yee2d_rb.cuh"
 
 using namespace mtb;
 
@@ -2093,6 +2094,13 @@ struct mtb_yee2d_plan {
     int cl_size = 0, cl_rows = 0;      // CTAs per cluster, rows per CTA
     size_t cl_bytes = 0;               // shared memory per CTA (with the sample staging)
     int cl_nmax = 0, cl_stage = 0;     // steps per launch; line samples staged
+    bool res = false;                  // resident kernel after the first step
+    bool rb_cl = false;                // it rounds as the cluster kernel does
+    DevBuf rb_work_d, rb_meta_d;       // its tile list (TM first), records
+    DevBuf rb_sync_d;                  // epoch flag per tile, then the neighbour lists
+    int n_rb[2] = {0, 0};              // TM, TE tiles
+    int rb_rw[2] = {0, 0}, rb_w[2] = {0, 0};   // rows per warp, warps per block
+    int rb_hits = 0;                   // room for line hits per warp
     DevBuf tb_work_d, tmaps_d;         // TB tile list (TM first), tensor maps
     DevBuf tb_meta_d, tb_prof_d;       // TB records, padded profiles
     int n_tb_tm = 0, n_tb_te = 0, tb_grid = 148;
@@ -2383,6 +2391,8 @@ extern "C" {
 
 static int cl_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs,
                          bool must);
+static int rb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs,
+                         const std::vector<mtb_line_sample> &lines);
 
 
 int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
@@ -2394,13 +2404,16 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
     *out = nullptr;
     if (n < 1 || !structs_in) return fail(MTB_INVALID_ARG, "need at least one structure");
     if (n_amp_cols < 0) return fail(MTB_INVALID_ARG, "n_amp_cols < 0");
-    // default (0) and variant 3: the temporally blocked kernels after the first
-    // step when every structure is eligible, else tiles; 2: tiles only
+    // default (0): after the first step, when every structure is eligible, the resident
+    // kernel where the tiles fit the GPU, else the temporally blocked kernels; 3: the
+    // temporally blocked ones; 4: small TM grids only (resident or the cluster kernel); 2: the
+    // one-step tiles only
     const int tv = tuning ? tuning->variant : 0;
     if (tv < 0 || tv > 4) return fail(MTB_INVALID_ARG, "2D variant %d not in 0..4", tv);
     const int variant = tv == 1 ? 1 : 2;
     bool want_tb = tv == 3 || tv == 0;
     bool want_cl = tv == 4 || tv == 0;
+    bool want_res = tv == 4 || tv == 0;
     int rows = (tuning && tuning->rows_per_warp > 0) ? tuning->rows_per_warp : 32;
     int wr = 1;
     if (variant == 2) {
@@ -2420,6 +2433,7 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
     if (ring_slot_elems < 0 || (ring_slot_elems & 3))
         return fail(MTB_INVALID_ARG, "ring_slot_elems must be a non-negative multiple of 4");
     std::vector<mtb_yee2d_struct> structs(structs_in, structs_in + n);
+    std::vector<mtb_line_sample> lines((size_t)n * MAXL);   // host copies, MAXL per structure
     int64_t n_work = 0;
     for (int s = 0; s < n; ++s) {
         mtb_yee2d_struct &S = structs[s];
@@ -2607,7 +2621,7 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
         if (S.n_lines > 0 && !S.lines)
             return fail(MTB_INVALID_ARG, "structure %d: null line sample array", s);
         if (S.n_lines > 0) {
-            mtb_line_sample ls[MAXL];
+            mtb_line_sample *ls = lines.data() + (size_t)s * MAXL;
             cudaError_t e = cudaMemcpy(ls, S.lines, sizeof(mtb_line_sample) * S.n_lines,
                                        cudaMemcpyDeviceToHost);
             if (e != cudaSuccess)
@@ -2655,6 +2669,8 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
         if (structs[s].te3 && structs[s].nlx[0]) p->te_nl = true;
     }
     for (int s = 0; s < n; ++s) want_tb = want_tb && tb_eligible(structs[s]);
+    for (int s = 0; s < n; ++s)
+        want_res = want_res && tb_eligible(structs[s]);
     for (int s = 0; s < n; ++s)
         want_cl = want_cl && structs[s].pol == MTB_TM && tb_eligible(structs[s]);
     int rc = p->dft.init(regions, n_regions, groups, n_groups, ring_slot_elems, slots);
@@ -2706,7 +2722,14 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
         mtb_yee2d_plan_destroy(p);
         return rc;
     }
-    if (want_tb && !p->cl && (rc = tb_setup_plan(p, structs))) {
+    // a plan of the cluster kernel (its one or two barriers a step cost 3.3-4.4 us) or of the
+    // temporally blocked kernels whose tiles fit the GPU stays resident instead
+    if (want_res && (p->cl || want_tb) && (rc = rb_setup_plan(p, structs, lines))) {
+        mtb_yee2d_plan_destroy(p);
+        return rc;
+    }
+    if (p->res) p->cl = false;
+    if (want_tb && !p->cl && !p->res && (rc = tb_setup_plan(p, structs))) {
         mtb_yee2d_plan_destroy(p);
         return rc;
     }
@@ -2979,6 +3002,200 @@ static int launch_cl(mtb_yee2d_plan *p, const float *amp_e, const float *amp_h, 
     return MTB_OK;
 }
 
+// kernel of a polarisation (0 TM, 1 TE, 2 TM rounding as the cluster kernel)
+static const void *rb_fn(int kind, int rw) {
+    if (kind == 1)
+        return rw == 1 ? (const void *)k_rb_resident<true, 1, false>
+                       : (const void *)k_rb_resident<true, 2, false>;
+    if (kind == 2)
+        return rw == 1 ? (const void *)k_rb_resident<false, 1, true>
+                       : (const void *)k_rb_resident<false, 2, true>;
+    return rw == 1 ? (const void *)k_rb_resident<false, 1, false>
+                   : (const void *)k_rb_resident<false, 2, false>;
+}
+
+// Output rows per resident tile: the fewest (at least RB_T, so that a halo never reaches
+// past the next tile) for which every tile of the polarisation gets an SM of its own; 0 if
+// there are too many. Tiles in place of the temporally blocked kernels' divide their
+// TB_OUTR rows (any: no such constraint).
+static int rb_resident_rows(const std::vector<mtb_yee2d_struct> &structs, int pol, int sms,
+                            bool any) {
+    for (int R = RB_T; R <= 2 * RB_WARPS - 2 * RB_T; ++R) {
+        if (!any && TB_OUTR % R != 0) continue;
+        int64_t n = 0;
+        for (const auto &S : structs)
+            if (S.pol == pol)
+                n += (int64_t)((S.nx + R - 1) / R) * ((S.pitch + RB_OUTC - 1) / RB_OUTC);
+        if (n <= sms) return R;
+    }
+    return 0;
+}
+static_assert(RB_OUTC == TB_OUTC && RB_T == TB_T && RB_C == TB_C, "one column grid, one depth");
+static_assert(2 * RB_WARPS - 2 * RB_T == TB_OUTR, "a whole block of the other is the largest tile");
+
+// Flags of the tile with output rows [r0, r0 + rows), columns [c0, c0 + RB_OUTC).
+static int rb_flags(const mtb_yee2d_struct &S, const mtb_line_sample *ls, int r0, int rows, int c0) {
+    // layer extents: rows [0, XL) and [XH, nx), columns [0, YL) and [YH, ny)
+    const int XL = std::max(S.xband[0], S.xband[2]), XH = std::min(S.xband[1], S.xband[3]);
+    const int YL = std::max(S.yband[0], S.yband[2]), YH = std::min(S.yband[1], S.yband[3]);
+    const int wr0 = r0 - RB_T, wr1 = r0 + rows + RB_T, wc0 = c0 - 4, wc1 = c0 - 4 + RB_C;
+    int f = 0;
+    if (wr0 < XL || wr1 > XH) f |= RBF_XL;
+    if (std::min(wc1, YL) > std::max(wc0, 0) || std::min(wc1, S.ny) > std::max(wc0, YH))
+        f |= RBF_YL;
+    // lean: the temporally blocked tile around it is (as tb_setup_plan decides)
+    const int b0 = r0 / TB_OUTR * TB_OUTR - TB_T, b1 = b0 + TB_R;
+    if (!(f & RBF_YL) && b0 >= std::max(XL, 1) && b1 <= std::min(XH, S.nx - 1) && wc0 >= 1 &&
+        wc1 <= S.ny - 1)
+        f |= RBF_LEAN;
+    for (const mtb_cells *c : {&S.src_e, &S.src_h1, &S.src_h2})
+        if (c->n > 0 && c->row_lo <= wr1 && c->row_hi >= wr0 - 1) f |= RBF_SRC;
+    for (int l = 0; l < S.n_lines; ++l) {
+        const mtb_line_sample &q = ls[l];
+        const bool t = q.kind == 0 ? (q.index >= r0 && q.index < r0 + rows && q.lo < c0 + RB_OUTC &&
+                                      q.hi > c0)
+                                   : (q.index >= c0 && q.index < c0 + RB_OUTC &&
+                                      q.lo < r0 + rows && q.hi > r0);
+        if (t) f |= RBF_LINES;
+    }
+    return f;
+}
+
+// Resident kernel: records, tile list (TM first, then TE), neighbours and flags. Taken when
+// the tiles of each polarisation fit the GPU at once, one block per SM (24 x 120 output
+// cells a tile at most: about 426 k cells); leaves p->res false otherwise. The line lies
+// where a second tile per SM would begin: below it a step costs 1.5-2.7 us here against
+// 3.3-4.3 us with launches of four steps or the cluster kernel; past it the blocks could
+// not all be resident, which their waits on one another need.
+static int rb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs,
+                         const std::vector<mtb_line_sample> &lines) {
+    const int n = (int)structs.size();
+    int dev = 0, sms = 0, coop = 0, rc;
+    MTB_CUDA_TRY(cudaGetDevice(&dev));
+    MTB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MTB_CUDA_TRY(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop || p->dft.slots > RB_SLOTS) return MTB_OK;
+    int R[2] = {0, 0}, max_lines = 0;
+    for (int pol = 0; pol < 2; ++pol) {
+        bool any = false;
+        for (const auto &S : structs) any = any || S.pol == (pol == 0 ? MTB_TM : MTB_TE);
+        if (!any) continue;
+        R[pol] = rb_resident_rows(structs, pol == 0 ? MTB_TM : MTB_TE, sms, p->cl);
+        if (!R[pol]) return MTB_OK;
+    }
+    for (const auto &S : structs) max_lines = std::max(max_lines, S.n_lines);
+    p->rb_hits = 2 * max_lines;
+    {   // shared-memory limits, once per process and device
+        static std::mutex mu;
+        static std::vector<int> done;
+        std::lock_guard<std::mutex> lock(mu);
+        if (std::find(done.begin(), done.end(), dev) == done.end()) {
+            for (int rw = 1; rw <= 2; ++rw) {
+                const auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
+                const int b = (int)rb_res_smem(RB_WARPS, rw, 2 * MAXL);
+                for (int kind = 0; kind < 3; ++kind)
+                    MTB_CUDA_TRY(cudaFuncSetAttribute(rb_fn(kind, rw), A, b));
+            }
+            done.push_back(dev);
+        }
+    }
+    std::vector<RbMeta> metas(n);
+    for (int s = 0; s < n; ++s) {
+        std::memset(&metas[s], 0, sizeof(RbMeta));
+        metas[s].s = structs[s];
+        std::memcpy(metas[s].lines, lines.data() + (size_t)s * MAXL,
+                    sizeof(mtb_line_sample) * structs[s].n_lines);
+    }
+    std::vector<int4> work;
+    std::vector<int> nb;
+    for (int pol = 0; pol < 2; ++pol) {
+        if (!R[pol]) continue;
+        p->rb_rw[pol] = R[pol] + 2 * RB_T <= RB_WARPS ? 1 : 2;
+        p->rb_w[pol] = (R[pol] + 2 * RB_T + p->rb_rw[pol] - 1) / p->rb_rw[pol];
+        const size_t w0 = work.size();
+        for (int s = 0; s < n; ++s) {
+            const mtb_yee2d_struct &S = structs[s];
+            if (S.pol != (pol == 0 ? MTB_TM : MTB_TE)) continue;
+            const int nr = (S.nx + R[pol] - 1) / R[pol], nc = (S.pitch + RB_OUTC - 1) / RB_OUTC;
+            const int t0 = (int)((work.size() - w0) / RB_WORK);
+            for (int a = 0; a < nr; ++a)
+                for (int c = 0; c < nc; ++c) {
+                    const int r0 = a * R[pol], c0 = c * RB_OUTC;
+                    const int rows = std::min(R[pol], S.nx - r0);
+                    work.push_back(make_int4(s, r0, c0,
+                                             rb_flags(S, metas[s].lines, r0, rows, c0)));
+                    work.push_back(make_int4(rows, 0, 0, 0));
+                    for (int k = 0; k < 9; ++k) {
+                        const int aa = a + k / 3 - 1, cc = c + k % 3 - 1;
+                        if (k == 4) continue;
+                        nb.push_back(aa >= 0 && aa < nr && cc >= 0 && cc < nc ? t0 + aa * nc + cc
+                                                                              : -1);
+                    }
+                }
+        }
+        p->n_rb[pol] = (int)((work.size() - w0) / RB_WORK);
+    }
+    std::vector<int> sync(nb.size() / 8, 0);
+    sync.insert(sync.end(), nb.begin(), nb.end());
+    if ((rc = p->rb_work_d.ensure(sizeof(int4) * work.size())) ||
+        (rc = p->rb_meta_d.ensure(sizeof(RbMeta) * metas.size())) ||
+        (rc = p->rb_sync_d.ensure(sizeof(int) * sync.size())))
+        return rc;
+    cudaError_t e = cudaMemcpy(p->rb_work_d.p, work.data(), sizeof(int4) * work.size(),
+                               cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(p->rb_meta_d.p, metas.data(), sizeof(RbMeta) * metas.size(),
+                       cudaMemcpyHostToDevice);
+    if (e == cudaSuccess)
+        e = cudaMemcpy(p->rb_sync_d.p, sync.data(), sizeof(int) * sync.size(),
+                       cudaMemcpyHostToDevice);
+    if (e != cudaSuccess)
+        return fail(MTB_CUDA_ERROR, "resident set-up: %s", cudaGetErrorString(e));
+    p->res = true;
+    p->rb_cl = p->cl;
+    return MTB_OK;
+}
+
+// n resident steps (never past the ring's end) from parity par, one launch per
+// polarisation; samples from ring slot `slot` on. The parity flips once per RB_T steps.
+static int launch_rb(mtb_yee2d_plan *p, const float *amp_e, const float *amp_h, int nc, int n,
+                     int slot, int par, cudaStream_t st) {
+    for (int pol = 0; pol < 2; ++pol) {
+        if (p->n_rb[pol] == 0) continue;
+        const int before = pol ? p->n_rb[0] : 0, total = p->n_rb[0] + p->n_rb[1];
+        RbCtx C;
+        C.meta = p->rb_meta_d.as<RbMeta>();
+        C.amp_e = amp_e;
+        C.amp_h = amp_h;
+        C.ncols = nc;
+        C.nsub = n;
+        C.ring = p->dft.ring_d.as<float>() + (size_t)slot * p->dft.slot_elems;
+        C.slot_elems = p->dft.slot_elems;
+        C.err = p->err_d.as<int>();
+        C.par = par;
+        C.work = p->rb_work_d.as<int4>() + (size_t)RB_WORK * before;
+        C.flags = p->rb_sync_d.as<int>() + before;
+        C.nb = p->rb_sync_d.as<int>() + total + 8 * (size_t)before;
+        C.hits = p->rb_hits;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        cfg.gridDim = dim3(p->n_rb[pol]);
+        cfg.blockDim = dim3(32 * p->rb_w[pol]);
+        cfg.dynamicSmemBytes = rb_res_smem(p->rb_w[pol], p->rb_rw[pol], p->rb_hits);
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        void *args[1] = {&C};
+        MTB_CUDA_TRY(cudaLaunchKernelExC(&cfg, rb_fn(pol == 1 ? 1 : p->rb_cl ? 2 : 0, p->rb_rw[pol]), args));
+        MTB_CHECK_LAUNCH();
+        ++p->last_launches;
+    }
+    return MTB_OK;
+}
+static int rb_flips(int n) { return ((n + RB_T - 1) / RB_T) & 1; }
+
 // Capture one ring flush (G steps from parity par0, then the contraction)
 // reading its coefficient and phase rows from the plan's staging buffer.
 static int build_flush_graph(mtb_yee2d_plan *p, int par0, int nc) {
@@ -2998,6 +3215,11 @@ static int build_flush_graph(mtb_yee2d_plan *p, int par0, int nc) {
             par ^= n & 1;
             s += n;
             continue;
+        }
+        if (p->res) {
+            rc = launch_rb(p, stage, stage + (size_t)G * nc, nc, G, 0, par, p->cap);
+            par ^= rb_flips(G);
+            break;
         }
         if (p->tb) {                             // TB launches of up to TB_T steps
             const int n = std::min(TB_T, G - s);
@@ -3053,9 +3275,10 @@ int mtb_yee2d_run(mtb_yee2d_plan *p, int64_t t0, int32_t k, const double *coef_e
     if (k == 0) return MTB_OK;
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
-    // the row march's bounded waits may have raised the error flag (the TB kernels' flag
-    // is read by mtb_yee2d_check, which the engine calls when it exports the state; the
-    // one-step tiles and the cluster kernel never wait)
+    // the row march's bounded waits may have raised the error flag (the TB and resident
+    // kernels' flag is read by mtb_yee2d_check, which the engine calls when it exports the
+    // state; the one-step
+    // tiles and the cluster kernel never wait)
     if (p->variant == 1 && (rc = mtb_yee2d_check(p, stream))) return rc;
     const int nc = std::max(p->n_cols, 1);
     const size_t per = (size_t)k * nc;
@@ -3110,6 +3333,26 @@ int mtb_yee2d_run(mtb_yee2d_plan *p, int64_t t0, int32_t k, const double *coef_e
                 return rc;
             if ((rc = p->timer.end(st))) return rc;
             p->par ^= n & 1;
+            s += n;
+            slot += n;
+            if (slot == G || s == k) {
+                if (p->dft.n_regions > 0) {
+                    if ((rc = p->dft.contract(s - slot, slot, st, &p->timer))) return rc;
+                    ++p->last_launches;
+                }
+                slot = 0;
+            }
+            continue;
+        }
+        if (p->res && !p->first) {
+            // resident: the rest of the ring (or of the run) in one launch
+            const int n = std::min(G - slot, k - s);
+            if ((rc = p->timer.begin(st, 0))) return rc;
+            if ((rc = launch_rb(p, ad + (size_t)s * nc, ad + per + (size_t)s * nc, nc, n, slot,
+                                p->par, st)))
+                return rc;
+            if ((rc = p->timer.end(st))) return rc;
+            p->par ^= rb_flips(n);
             s += n;
             slot += n;
             if (slot == G || s == k) {
@@ -3223,6 +3466,9 @@ void mtb_yee2d_plan_destroy(mtb_yee2d_plan *p) {
         if (p->gexec[q]) cudaGraphExecDestroy(p->gexec[q]);
     if (p->cap) cudaStreamDestroy(p->cap);
     p->stage_d.release();
+    p->rb_work_d.release();
+    p->rb_meta_d.release();
+    p->rb_sync_d.release();
     p->tb_work_d.release();
     p->tmaps_d.release();
     p->tb_meta_d.release();
