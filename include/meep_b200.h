@@ -625,6 +625,13 @@ int mtb_unpack_ratio(const float *box, const float *den, int64_t n0, int64_t n1,
                      int64_t off1, int64_t off2, float *dst, int64_t s0,
                      int64_t s1, void *stream);
 
+/* eps and 1/eps boxes (n0 rows of `pitch` floats, zero past column n1) of a dense n0 x n1
+ * array, in one pass. */
+int mtb_pack_eps(const float *src, int64_t n0, int64_t n1, int64_t pitch, float *eps,
+                 float *inv, void *stream);
+/* Zero `count` device buffers (addresses bufs[k], n[k] floats each; host arrays). */
+int mtb_zero(const uint64_t *bufs, const int64_t *n, int32_t count, void *stream);
+
 /* Count entries of x (n floats) whose |x| > 0 where mask_row (per leading
  * index, n0 entries) and mask_col (per last index) are both zero -- used to
  * check CPML memory is zero outside the absorbing layers on import. */

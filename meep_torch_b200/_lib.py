@@ -163,6 +163,8 @@ SIGNATURES = {
     "mtb_pack": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, vp,
                            C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                            C.c_int64, C.c_int64, vp]),
+    "mtb_pack_eps": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, vp, vp, vp]),
+    "mtb_zero": (C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_int64), C.c_int32, vp]),
     "mtb_unpack": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                              C.c_int64, C.c_int64, C.c_int64, vp, C.c_int64, C.c_int64, vp]),
     "mtb_unpack_ratio": (C.c_int, [vp, vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
@@ -225,6 +227,13 @@ def check(rc: int, what: str = ""):
     if rc == MTB_UNSUPPORTED:
         raise MtbUnsupported(msg)
     raise MtbError(f"[status {rc}] {msg}")
+
+
+def zero(lib, bufs, stream: int):
+    """Zero the float buffers ``bufs`` (contiguous device tensors) on ``stream``."""
+    n = len(bufs)
+    check(lib.mtb_zero((C.c_uint64 * n)(*[t.data_ptr() for t in bufs]),
+                       (C.c_int64 * n)(*[t.numel() for t in bufs]), n, stream), "mtb_zero")
 
 
 def ptr(t) -> int:

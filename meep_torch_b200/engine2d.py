@@ -835,17 +835,10 @@ class Engine2D:
     def reset(self):
         """Zero every field, CPML and accumulator buffer (both ping-pong halves)
         with the library's own fill kernel -- a fresh t = 0 run of the same batch."""
-        for it in self.items:
-            bufs = [*it.box["main"], *it.box["x"], *it.box["y"]] + \
-                [t for p in it.box["psi"] for t in p] + list(it.accs) + \
-                list(it.box.get("pol", [])) + list(it.box.get("pol_x", [])) + \
-                list(it.box.get("pol_y", []))
-            for t in bufs:
-                n = t.numel()
-                if n == 0:
-                    continue
-                L.check(self.lib.mtb_pack(0, 0, 0, 0, 0, 0, L.ptr(t), 1, 1, n, n, n, 0, 0, 0,
-                                          self._sptr()), "reset")
+        L.zero(self.lib, [t for it in self.items for t in (
+            *it.box["main"], *it.box["x"], *it.box["y"], *(t for p in it.box["psi"] for t in p),
+            *it.accs, *it.box.get("pol", ()), *it.box.get("pol_x", ()),
+            *it.box.get("pol_y", ()))], self._sptr())
 
     def set_eps(self, b: int, eps: torch.Tensor):
         """Replace structure b's permittivity in place (a TM structure without
@@ -857,9 +850,9 @@ class Engine2D:
               "poles or an explicit first-step Ez only")
         _need(tuple(eps.shape) == (it.nx, it.ny), f"set_eps: eps shape {tuple(eps.shape)} "
               f"!= {(it.nx, it.ny)}")
-        e = eps.to(device=self.device, dtype=torch.float32)
-        it.box["eps_a"].copy_(self._pack(e, it.nx, it.pitch))
-        it.box["inv_a"].copy_(self._pack(torch.reciprocal(e), it.nx, it.pitch))
+        e = eps.detach().to(device=self.device, dtype=torch.float32).contiguous()
+        L.check(self.lib.mtb_pack_eps(L.ptr(e), it.nx, it.ny, it.pitch, L.ptr(it.box["eps_a"]),
+                                      L.ptr(it.box["inv_a"]), self._sptr()), "set_eps")
 
     def _live_buffers(self, b: int):
         """The buffers of structure b the next step reads: fields, CPML memory, pole

@@ -428,12 +428,8 @@ class Engine3D:
 
     def reset(self):
         """Zero every field, CPML and accumulator buffer (t = 0 again)."""
-        bufs = [t for p in self.box.values() for t in p] + list(self.accs) + \
-            [t for p in getattr(self, "pol_box", {}).values() for t in p]
-        for t in bufs:
-            n = t.numel()
-            L.check(self.lib.mtb_pack(0, 0, 0, 0, 0, 0, L.ptr(t), 1, 1, n, n, n, 0, 0, 0,
-                                      self._sptr()), "reset")
+        L.zero(self.lib, [t for p in self.box.values() for t in p] + list(self.accs) +
+               [t for p in getattr(self, "pol_box", {}).values() for t in p], self._sptr())
 
     def set_timing(self, on: bool = True):
         L.check(self.lib.mtb_yee3d_set_timing(self.plan, 1 if on else 0), "set_timing")
