@@ -156,6 +156,7 @@ struct DftState {
     int total_nf = 0;                      // sum of nf
     // device
     DevBuf regions_d, blk_start_d, blk_region_d, phase_d, ring_d;
+    DevBuf freq_dt_d;                      // {frequency, dt} of every phase column
     PinnedPair phase_h;
     int64_t slot_elems = 0;
     int slots = 0;                         // ring depth K
@@ -164,7 +165,7 @@ struct DftState {
 
     int init(const mtb_dft_region *regions, int n_regions, const mtb_phase_group *groups,
              int n_groups, int64_t slot_elems, int slots);
-    // Fill the phase table for steps [t0, t0+k) and upload it on `st`.
+    // The phase table of steps [t0, t0+k), on `st`.
     int upload_phases(int64_t t0, int k, cudaStream_t st);
     // Fold ring slots [0, n) (steps t_first .. t_first+n-1, relative row
     // `row0` of the uploaded table, or of `phase_base` when given) into the
