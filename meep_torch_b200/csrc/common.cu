@@ -180,95 +180,179 @@ static int grid_for(int64_t total, int threads = 256) {
 constexpr int KMAX = 64;       // deepest ring supported by the contraction
 constexpr int CT = 256;        // channels per contraction block
 
-// One block folds CT channels of one region (region of the block from a
-// per-block table). Phase values of the region's (group, toff) are staged
-// in shared memory, sP[s * nf + f] = (Re, Im); each thread keeps NFC
-// frequencies of its channel in registers and streams its n ring samples.
+// A chunk is CT channels of one region (the region of a chunk from a per-chunk table); a
+// block folds a contiguous range of chunks. Phase values of a region's (group, toff) are
+// staged in shared memory, frequency by frequency (sP[(f - fa) * (n + 2) + s] = (Re, Im);
+// the two spare columns spread the staging stores over the banks), and staged again only where the range enters a region of another group or time offset.
+//
+// What bounds it: memory, given enough loads in flight. A block per chunk spent its time in
+// the chain table -> region -> phases -> samples -> accumulators, one frequency after the
+// other (bends batch, 5.3 M channels: 285 us per 32-step flush, 3.2 TB/s). Now a block's
+// first chain serves all of its chunks, and the accumulators of NFC frequencies are loaded
+// with the samples, the next NFC before the last ones are stored; the region sits in shared
+// memory, since in registers it spilled. Now 214 us (4.2 TB/s; 64 designs: 203 ->
+// 151 us, 256^3 flux faces 59 -> 40 us, 24 frequencies of a flux line 6.8 -> 5.5 us).
 constexpr int NFC = 4;
 constexpr int KFULL = 32;      // ring depth with a fully unrolled contraction (the default)
-__global__ void __launch_bounds__(CT, 4) k_dft_contract(
+constexpr int SB = 16;         // samples in flight at other depths
+__global__ void __launch_bounds__(CT, 3) k_dft_contract(
     const mtb_dft_region *__restrict__ regions, const int *__restrict__ blk_region,
     const int64_t *__restrict__ blk_start, const int *__restrict__ group_nf,
     const int *__restrict__ group_off, int total_nf, const float *__restrict__ phase, int row0,
-    int n, const float *__restrict__ ring, int64_t slot_elems) {
-    extern __shared__ float2 sP[];
-    const int64_t b = blockIdx.x;
-    const int rg = blk_region[b];
-    const mtb_dft_region R = regions[rg];
-    const int nf = group_nf[R.group];
-    const int foff = group_off[R.group];
-    const int sel = (R.toff == 2) ? 2 : 0;
-    for (int e = threadIdx.x; e < n * nf; e += CT) {
-        const int s = e / nf, f = e - s * nf;
-        const float *p = phase + ((int64_t)(row0 + s) * total_nf + foff + f) * 4 + sel;
-        sP[e] = make_float2(p[0], p[1]);
-    }
-    __syncthreads();
-    const int64_t ch = (b - blk_start[rg]) * CT + threadIdx.x;
-    const int64_t nch = (int64_t)R.rows * R.cols;
-    if (ch >= nch) return;
-    // frequencies [fa, fb) of this block row (small channel counts split the
-    // frequency loop over gridDim.y block rows; each sum is formed as without it)
-    const int per = (nf + gridDim.y - 1) / gridDim.y;
-    const int fa = blockIdx.y * per, fb = min(nf, fa + per);
-    if (fa >= fb) return;
-    const int r = (int)(ch / R.cols), c = (int)(ch - (int64_t)r * R.cols);
-    const float *xa = ring + R.ring_a + (int64_t)r * R.ring_pitch + c;
-    const float *xb = (R.ring_b >= 0) ? ring + R.ring_b + (int64_t)r * R.ring_pitch + c : nullptr;
-    float *acc = R.acc;
-    const int64_t base = (int64_t)r * R.acc_pitch + c;
-    if (n == KFULL) {
-        // a whole ring: every sample of the channel in flight at once
-        float x[KFULL];
-#pragma unroll
-        for (int s = 0; s < KFULL; ++s) x[s] = __ldg(xa + s * slot_elems);
-        if (xb) {
-#pragma unroll
-            for (int s = 0; s < KFULL; ++s) x[s] = 0.5f * (x[s] + __ldg(xb + s * slot_elems));
-        }
-        for (int f = fa; f < fb; ++f) {
-            float re = 0.f, im = 0.f;
-#pragma unroll
-            for (int s = 0; s < KFULL; ++s) {
-                const float2 p = sP[s * nf + f];
-                re = fmaf(p.x, x[s], re);
-                im = fmaf(p.y, x[s], im);
+    int n, const float *__restrict__ ring, int64_t slot_elems, int64_t n_chunks) {
+    extern __shared__ float4 sP4[];
+    float2 *sP = reinterpret_cast<float2 *>(sP4);
+    const int64_t per = (n_chunks + gridDim.x - 1) / gridDim.x;
+    const int64_t c0 = blockIdx.x * per, c1 = min(n_chunks, c0 + per);
+    __shared__ mtb_dft_region R;             // (in registers it spills)
+    int rg = -1, staged = -1, fa = 0, fb = 0;
+    int64_t first = 0;
+    for (int64_t b = c0; b < c1; ++b) {
+        const int q = blk_region[b];
+        if (q != rg) {
+            rg = q;
+            first = blk_start[rg];
+            __syncthreads();                 // the last chunk's readers are done
+            for (int e = threadIdx.x; e < (int)(sizeof(R) / 4); e += CT)
+                reinterpret_cast<int *>(&R)[e] = reinterpret_cast<const int *>(regions + rg)[e];
+            __syncthreads();
+            const int nf = group_nf[R.group];
+            // frequencies [fa, fb) of this block row (small channel counts split the
+            // frequency loop over gridDim.y block rows; each sum is formed as without it)
+            const int pf = (nf + gridDim.y - 1) / gridDim.y;
+            fa = blockIdx.y * pf;
+            fb = min(nf, fa + pf);
+            const int sel = (R.toff == 2) ? 2 : 0;
+            if (staged != 2 * R.group + (sel >> 1)) {
+                staged = 2 * R.group + (sel >> 1);
+                const float *p0 = phase + ((int64_t)row0 * total_nf + group_off[R.group]) * 4 + sel;
+                for (int e = threadIdx.x; e < n * (fb - fa); e += CT) {
+                    const int s = e / (fb - fa), f = e - s * (fb - fa);
+                    const float *p = p0 + ((int64_t)s * total_nf + fa + f) * 4;
+                    sP[f * (n + 2) + s] = make_float2(p[0], p[1]);
+                }
+                __syncthreads();
             }
-            acc[R.re_off + f * R.f_stride + base] += re;
-            acc[R.im_off + f * R.f_stride + base] += im;
         }
-        return;
-    }
-    for (int f0 = fa; f0 < fb; f0 += NFC) {
-        float *pr[NFC], *pi[NFC];
-        float re[NFC], im[NFC];
+        const int64_t ch = (b - first) * CT + threadIdx.x;
+        if (fa >= fb || ch >= (int64_t)R.rows * R.cols) continue;
+        const int r = (int)(ch / R.cols), c = (int)(ch - (int64_t)r * R.cols);
+        const float *xa = ring + R.ring_a + (int64_t)r * R.ring_pitch + c;
+        const float *xb = (R.ring_b >= 0) ? ring + R.ring_b + (int64_t)r * R.ring_pitch + c : nullptr;
+        float *pre = R.acc + R.re_off + (int64_t)r * R.acc_pitch + c;
+        float *pim = R.acc + R.im_off + (int64_t)r * R.acc_pitch + c;
+        const int64_t fs = R.f_stride;
+        if (n == KFULL) {
+            // a whole ring: every sample of the channel in flight at once
+            float x[KFULL], ore[NFC], oim[NFC];
 #pragma unroll
-        for (int q = 0; q < NFC; ++q) {
-            const int f = min(f0 + q, fb - 1);
-            pr[q] = acc + R.re_off + f * R.f_stride + base;
-            pi[q] = acc + R.im_off + f * R.f_stride + base;
-            re[q] = 0.f;
-            im[q] = 0.f;
-        }
-#pragma unroll 4
-        for (int s = 0; s < n; ++s) {
-            float x = xa[s * slot_elems];
-            if (xb) x = 0.5f * (x + xb[s * slot_elems]);
-            const float2 *ps = sP + s * nf + f0;
+            for (int s = 0; s < KFULL; ++s) x[s] = __ldg(xa + s * slot_elems);
 #pragma unroll
-            for (int q = 0; q < NFC; ++q) {
-                if (f0 + q < fb) {
-                    const float2 p = ps[q];
-                    re[q] = fmaf(p.x, x, re[q]);
-                    im[q] = fmaf(p.y, x, im[q]);
+            for (int k = 0; k < NFC; ++k) {
+                const int64_t o = min(fa + k, fb - 1) * fs;
+                ore[k] = pre[o];
+                oim[k] = pim[o];
+            }
+            if (xb) {
+#pragma unroll
+                for (int s = 0; s < KFULL; ++s) x[s] = 0.5f * (x[s] + __ldg(xb + s * slot_elems));
+            }
+            for (int f0 = fa; f0 < fb; f0 += NFC) {
+                float re[NFC], im[NFC];
+#pragma unroll
+                for (int k = 0; k < NFC; ++k) {
+                    re[k] = 0.f;
+                    im[k] = 0.f;
+                    if (f0 + k < fb) {
+                        const float4 *pf = sP4 + (f0 - fa + k) * (KFULL / 2 + 1);
+#pragma unroll
+                        for (int s = 0; s < KFULL; s += 2) {
+                            const float4 p = pf[s / 2];
+                            re[k] = fmaf(p.x, x[s], re[k]);
+                            im[k] = fmaf(p.y, x[s], im[k]);
+                            re[k] = fmaf(p.z, x[s + 1], re[k]);
+                            im[k] = fmaf(p.w, x[s + 1], im[k]);
+                        }
+                        re[k] += ore[k];
+                        im[k] += oim[k];
+                    }
+                }
+                if (f0 + NFC < fb) {
+#pragma unroll
+                    for (int k = 0; k < NFC; ++k) {
+                        const int64_t o = min(f0 + NFC + k, fb - 1) * fs;
+                        ore[k] = pre[o];
+                        oim[k] = pim[o];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < NFC; ++k) {
+                    if (f0 + k < fb) {
+                        pre[(f0 + k) * fs] = re[k];
+                        pim[(f0 + k) * fs] = im[k];
+                    }
                 }
             }
+            continue;
         }
+        for (int f0 = fa; f0 < fb; f0 += NFC) {
+            float *pr[NFC], *pi[NFC];
+            float re[NFC], im[NFC];
 #pragma unroll
-        for (int q = 0; q < NFC; ++q) {
-            if (f0 + q < fb) {
-                *pr[q] += re[q];
-                *pi[q] += im[q];
+            for (int k = 0; k < NFC; ++k) {
+                const int64_t o = min(f0 + k, fb - 1) * fs;
+                pr[k] = pre + o;
+                pi[k] = pim + o;
+                re[k] = 0.f;
+                im[k] = 0.f;
+            }
+            // blocks of SB samples in flight at once (even n: the phases as float4), the rest
+            // one by one
+            const int nb = (n & 1) ? 0 : n / SB * SB;
+            for (int s0 = 0; s0 < nb; s0 += SB) {
+                float x[SB];
+#pragma unroll
+                for (int i = 0; i < SB; ++i) x[i] = xa[(s0 + i) * slot_elems];
+                if (xb) {
+#pragma unroll
+                    for (int i = 0; i < SB; ++i) x[i] = 0.5f * (x[i] + xb[(s0 + i) * slot_elems]);
+                }
+#pragma unroll
+                for (int k = 0; k < NFC; ++k) {
+                    if (f0 + k < fb) {
+                        const float4 *pf = reinterpret_cast<const float4 *>(
+                            sP + (f0 - fa + k) * (n + 2) + s0);
+#pragma unroll
+                        for (int i = 0; i < SB; i += 2) {
+                            const float4 p = pf[i / 2];
+                            re[k] = fmaf(p.x, x[i], re[k]);
+                            im[k] = fmaf(p.y, x[i], im[k]);
+                            re[k] = fmaf(p.z, x[i + 1], re[k]);
+                            im[k] = fmaf(p.w, x[i + 1], im[k]);
+                        }
+                    }
+                }
+            }
+#pragma unroll 4
+            for (int s = nb; s < n; ++s) {
+                float x = xa[s * slot_elems];
+                if (xb) x = 0.5f * (x + xb[s * slot_elems]);
+                const float2 *ps = sP + (f0 - fa) * (n + 2) + s;
+#pragma unroll
+                for (int k = 0; k < NFC; ++k) {
+                    if (f0 + k < fb) {
+                        const float2 p = ps[k * (n + 2)];
+                        re[k] = fmaf(p.x, x, re[k]);
+                        im[k] = fmaf(p.y, x, im[k]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < NFC; ++k) {
+                if (f0 + k < fb) {
+                    *pr[k] += re[k];
+                    *pi[k] += im[k];
+                }
             }
         }
     }
@@ -477,12 +561,11 @@ int DftState::contract(int row0, int n, cudaStream_t st, LaunchTimer *tm,
     if (n_regions == 0 || n <= 0 || n_blocks == 0) return MTB_OK;
     int maxnf = 1;
     for (int g = 0; g < n_groups; ++g) maxnf = std::max(maxnf, group_nf[g]);
-    const size_t smem = sizeof(float2) * (size_t)n * maxnf;
     static bool attr_set = false;
     if (!attr_set) {
         MTB_CUDA_TRY(cudaFuncSetAttribute(k_dft_contract,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          sizeof(float2) * KMAX * 256));
+                                          sizeof(float2) * (KMAX + 2) * 256));
         attr_set = true;
     }
     const int *gd = reinterpret_cast<const int *>(blk_start_d.as<int64_t>() + (n_regions + 1));
@@ -493,11 +576,14 @@ int DftState::contract(int row0, int n, cudaStream_t st, LaunchTimer *tm,
     // frequencies each) until the launch has about 2^17 threads
     const int64_t want = ((int64_t)1 << 17) / std::max<int64_t>(n_blocks * CT, 1);
     const int fsplit = (int)std::max<int64_t>(1, std::min<int64_t>(want, (maxnf + 3) / 4));
-    k_dft_contract<<<dim3((unsigned)n_blocks, fsplit), CT, smem, st>>>(
+    const size_t smem = sizeof(float2) * (size_t)(n + 2) * ((maxnf + fsplit - 1) / fsplit);
+    // enough blocks for 16 per SM, then more chunks per block
+    const int64_t nb = std::min<int64_t>(n_blocks, 148 * 16);
+    k_dft_contract<<<dim3((unsigned)nb, fsplit), CT, smem, st>>>(
         regions_d.as<mtb_dft_region>(), blk_region_d.as<int>(), blk_start_d.as<int64_t>(), gd,
         gd + (n_groups + 1), total_nf, phase_base ? phase_base : phase_d.as<float>(), row0, n,
         ring_d.as<float>(),
-        slot_elems);
+        slot_elems, n_blocks);
     MTB_CHECK_LAUNCH();
     if (tm && (rc = tm->end(st))) return rc;
     return MTB_OK;

@@ -3498,7 +3498,8 @@ __global__ void k_dft_contract(const mtb_dft_region *__restrict__ regions,
                                const int64_t *__restrict__ blk_start,
                                const int *__restrict__ group_nf, const int *__restrict__ group_off,
                                int total_nf, const float *__restrict__ phase, int row0, int n,
-                               const float *__restrict__ ring, int64_t slot_elems);
+                               const float *__restrict__ ring, int64_t slot_elems,
+                               int64_t n_chunks);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[MTB_NOALLOC_SCRATCH_BYTES];
 constexpr int NA_MAX_DEV = 64;
@@ -3780,7 +3781,7 @@ extern "C" int mtb_yee2d_run_noalloc(const mtb_yee2d_struct *s, const mtb_dft_re
                                           (int)smem_te()));
         MTB_CUDA_TRY(cudaFuncSetAttribute(k_dft_contract,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)(sizeof(float2) * 64 * 256)));
+                                          (int)(sizeof(float2) * 66 * 256)));
         g_noalloc_dev[dev] = static_cast<unsigned char *>(p);
     }
     unsigned char *base = g_noalloc_dev[dev];
@@ -3891,9 +3892,10 @@ extern "C" int mtb_yee2d_run_noalloc(const mtb_yee2d_struct *s, const mtb_dft_re
             first = false;
             ++slot;
             if ((slot == ring_slots || q == n - 1) && n_regions > 0 && n_blocks > 0) {
-                k_dft_contract<<<(unsigned)n_blocks, NA_CT, sizeof(float2) * slot * maxnf, st>>>(
+                k_dft_contract<<<(unsigned)std::min<int64_t>(n_blocks, 148 * 16), NA_CT,
+                                 sizeof(float2) * (slot + 2) * maxnf, st>>>(
                     dReg, dBlk, dBs, dGnf, dGoff, total_nf, dPhase, q + 1 - slot, slot, dRing,
-                    ring_slot_elems);
+                    ring_slot_elems, n_blocks);
                 MTB_CHECK_LAUNCH();
                 slot = 0;
             } else if (slot == ring_slots || q == n - 1) {
