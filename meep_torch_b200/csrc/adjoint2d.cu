@@ -50,9 +50,11 @@ __device__ __forceinline__ void stv(float *p, const float (&v)[4]) {
 // (every thread of the block reads them for each of its cells).
 __device__ __forceinline__ const mtb_line_sample *stage_lines(const mtb_yee2d_struct &S,
                                                               mtb_line_sample *sl) {
+    pdl_next();
     const int t = threadIdx.y * 32 + threadIdx.x;
     if (t < S.n_lines) sl[t] = S.lines[t];
     __syncthreads();
+    pdl_wait();
     return sl;
 }
 
@@ -349,6 +351,8 @@ __device__ __forceinline__ void adj_tm_ez_cell(const mtb_yee2d_struct &S,
 __global__ void __launch_bounds__(32 * AROWS) k_adj_tm_ez(const __grid_constant__ mtb_yee2d_struct S,
                                                           const __grid_constant__ mtb_adj2d_buffers B,
                                                           int cpar) {
+    pdl_next();
+    pdl_wait();
     adj_tm_ez_cell(S, B, blockIdx.y * AROWS + threadIdx.y,
                   (blockIdx.x * 32 + threadIdx.x) * 4, cpar);
 }
@@ -572,6 +576,8 @@ __device__ __forceinline__ void adj_te_hz_cell(const mtb_yee2d_struct &S,
 
 __global__ void __launch_bounds__(32 * AROWS) k_adj_te_hz(const __grid_constant__ mtb_yee2d_struct S,
                                                           const __grid_constant__ mtb_adj2d_buffers B) {
+    pdl_next();
+    pdl_wait();
     adj_te_hz_cell(S, B, blockIdx.y * AROWS + threadIdx.y,
                   (blockIdx.x * 32 + threadIdx.x) * 4);
 }
@@ -648,6 +654,10 @@ static int adjoint_chunk(mtb_yee2d_adjoint *p, int k, const float *rec, int64_t 
                 MTB_CUDA_TRY(cudaMemcpyAsync(p->b.g_cut[a][1], p->b.g_cut[a][0],
                                              sizeof(float) * (a ? S.ny : S.nx),
                                              cudaMemcpyDeviceToDevice, st));
+    // The first launch of the chunk is an ordinary one: the chunk's sample adjoints and its
+    // forward record, which the kernels read through the read-only path, are complete behind
+    // it. The others may start ahead of their
+    // predecessor's end (replayed from a graph this gained little: 10 us a step either way).
     for (int q = k - 1; q >= 0; --q) {
         const float *radj = radj_of(q);
         const float *rq = rec_of(q);
@@ -656,27 +666,26 @@ static int adjoint_chunk(mtb_yee2d_adjoint *p, int k, const float *rec, int64_t 
                 k_adj_tm_e<<<grid, blk, 0, st>>>(S, p->b, radj, rq + rec_offset[0], q & 1);
                 MTB_CHECK_LAUNCH();
             }
-            k_adj_tm_h<<<grid, blk, 0, st>>>(S, p->b, radj);
-            MTB_CHECK_LAUNCH();
+            if ((rc = launch_pdl(k_adj_tm_h, grid, blk, st, S, p->b, radj))) return rc;
             if (q > 0)
-                k_adj_tm_eze<<<grid, blk, 0, st>>>(S, p->b, radj_of(q - 1),
-                                                   rec_of(q - 1) + rec_offset[0], (q - 1) & 1);
+                rc = launch_pdl(k_adj_tm_eze, grid, blk, st, S, p->b, radj_of(q - 1),
+                                rec_of(q - 1) + rec_offset[0], (q - 1) & 1);
             else
-                k_adj_tm_ez<<<grid, blk, 0, st>>>(S, p->b, 0);
-            MTB_CHECK_LAUNCH();
+                rc = launch_pdl(k_adj_tm_ez, grid, blk, st, S, p->b, 0);
         } else {
             if (q == k - 1) {
                 k_adj_te_h<<<grid, blk, 0, st>>>(S, p->b, radj);
                 MTB_CHECK_LAUNCH();
             }
-            k_adj_te_e<<<grid, blk, 0, st>>>(S, p->b, radj, rq + rec_offset[0], rq + rec_offset[1]);
-            MTB_CHECK_LAUNCH();
+            if ((rc = launch_pdl(k_adj_te_e, grid, blk, st, S, p->b, radj, rq + rec_offset[0],
+                                 rq + rec_offset[1])))
+                return rc;
             if (q > 0)
-                k_adj_te_hzh<<<grid, blk, 0, st>>>(S, p->b, radj_of(q - 1));
+                rc = launch_pdl(k_adj_te_hzh, grid, blk, st, S, p->b, radj_of(q - 1));
             else
-                k_adj_te_hz<<<grid, blk, 0, st>>>(S, p->b);
-            MTB_CHECK_LAUNCH();
+                rc = launch_pdl(k_adj_te_hz, grid, blk, st, S, p->b);
         }
+        if (rc) return rc;
         p->last_launches += (q == k - 1) ? 3 : 2;
     }
     return MTB_OK;

@@ -71,7 +71,11 @@ __global__ void k_adj3_inject(const mtb_yee3d_struct *__restrict__ SS,
                               const float *__restrict__ radj, mtb_adj3d_buffers B) {
     const mtb_yee3d_struct &S = *SS;
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= pstart[n_planes]) return;
+    pdl_next();
+    if (e >= pstart[n_planes]) {
+        pdl_wait();
+        return;
+    }
     int lo = 0, hi = n_planes - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -86,6 +90,7 @@ __global__ void k_adj3_inject(const mtb_yee3d_struct *__restrict__ SS,
     if (axis == 0) { i = index; j = a; k = b; }
     else if (axis == 1) { i = a; j = index; k = b; }
     else { i = a; j = b; k = index; }
+    pdl_wait();                          // the descriptor and plane tables are constant
     atomicAdd(B.g[comp] + ((int64_t)i * S.ny + j) * S.zpitch + k,
               radj[S.plane_ring_off[lo] + p]);
 }
@@ -277,7 +282,9 @@ __global__ void __launch_bounds__(3 * A3_T, 2) k_adj3_fe(const __grid_constant__
                                                         const float *__restrict__ en,
                                                         const float *__restrict__ eo,
                                                         int64_t rec_comp) {
+    pdl_next();
     const A3Cell c(P);
+    pdl_wait();
     if (threadIdx.y == 0) a3_e<0, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
     else if (threadIdx.y == 1) a3_e<1, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
     else a3_e<2, FIN, FIN, MODE>(P, c, en, eo, rec_comp);
@@ -360,7 +367,9 @@ __device__ __forceinline__ void a3_h(const Adj3 &P, const A3Cell &c) {
 }
 
 __global__ void __launch_bounds__(3 * A3_T, 2) k_adj3_h(const __grid_constant__ Adj3 P) {
+    pdl_next();
     const A3Cell c(P);
+    pdl_wait();
     if (threadIdx.y == 0) a3_h<0>(P, c);
     else if (threadIdx.y == 1) a3_h<1>(P, c);
     else a3_h<2>(P, c);
@@ -368,7 +377,9 @@ __global__ void __launch_bounds__(3 * A3_T, 2) k_adj3_h(const __grid_constant__ 
 
 // The last step's fin (gE only).
 __global__ void __launch_bounds__(3 * A3_T) k_adj3_fin(const __grid_constant__ Adj3 P) {
+    pdl_next();
     const A3Cell c(P);
+    pdl_wait();
     const int C = threadIdx.y;
     float ge[4];
     zz(ge);
@@ -382,7 +393,9 @@ __global__ void __launch_bounds__(3 * A3_T) k_adj3_fin(const __grid_constant__ A
 // g_eps += the run's sums of each component's eps_c adjoint, divided by eps_c, at the two
 // cells of its Yee average.
 __global__ void __launch_bounds__(A3_T) k_adj3_eps(const __grid_constant__ Adj3 P) {
+    pdl_next();
     const A3Cell c(P);
+    pdl_wait();
     if (!c.act) return;
     const int i = c.i, j = c.j, ZP = P.zp;
     const uint32_t g = c.g, NYZ = (uint32_t)P.ny * ZP;
@@ -553,40 +566,37 @@ int mtb_yee3d_adjoint_run(mtb_yee3d_adjoint *p, int64_t t0, int32_t k, const flo
     const dim3 blk(A3_T, 3);
     const dim3 grid((unsigned)(((int64_t)A.ny * (A.zp / 4) + A3_T - 1) / A3_T), A.nx);
     const int mode = (A.dmp[0][0] ? 1 : 0) | (A.np > 0 ? 2 : 0);
+    // The first launch of the chunk is an ordinary one: the chunk's sample adjoints, which the
+    // kernels read through the read-only path, are complete behind it.
+    bool first = true;
+    auto go = [&](auto kernel, dim3 g, dim3 b, auto... args) -> int {
+        if (!first) return launch_pdl(kernel, g, b, st, args...);
+        first = false;
+        kernel<<<g, b, 0, st>>>(args...);
+        MTB_CHECK_LAUNCH();
+        return MTB_OK;
+    };
     auto inject = [&](int q) -> int {
         if (p->n_samples == 0) return MTB_OK;
         const float *radj = p->dft.ring_d.as<float>() + (size_t)q * p->dft.slot_elems;
-        k_adj3_inject<<<(unsigned)((p->n_samples + 255) / 256), 256, 0, st>>>(
-            p->s_d.as<mtb_yee3d_struct>(), p->pstart_d.as<int64_t>(), p->n_planes, radj, A.b);
-        MTB_CHECK_LAUNCH();
         ++p->last_launches;
-        return MTB_OK;
+        return go(k_adj3_inject, (unsigned)((p->n_samples + 255) / 256), 256,
+                  p->s_d.as<mtb_yee3d_struct>(), p->pstart_d.as<int64_t>(), p->n_planes, radj, A.b);
     };
     if ((rc = inject(k - 1))) return rc;
     for (int q = k - 1; q >= 0; --q) {
         const float *en = rec + (size_t)(q + 1) * rec_slot_stride;
         const float *eo = rec + (size_t)q * rec_slot_stride;
+        decltype(&k_adj3_fe<false, 0>) fe[8] = {
+            k_adj3_fe<false, 0>, k_adj3_fe<false, 1>, k_adj3_fe<false, 2>, k_adj3_fe<false, 3>,
+            k_adj3_fe<true, 0>,  k_adj3_fe<true, 1>,  k_adj3_fe<true, 2>,  k_adj3_fe<true, 3>};
         const bool fin = q < k - 1;
-        switch (mode + (fin ? 4 : 0)) {
-            case 0: k_adj3_fe<false, 0><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 1: k_adj3_fe<false, 1><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 2: k_adj3_fe<false, 2><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 3: k_adj3_fe<false, 3><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 4: k_adj3_fe<true, 0><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 5: k_adj3_fe<true, 1><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            case 6: k_adj3_fe<true, 2><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-            default: k_adj3_fe<true, 3><<<grid, blk, 0, st>>>(A, en, eo, rec_comp_stride); break;
-        }
-        MTB_CHECK_LAUNCH();
-        k_adj3_h<<<grid, blk, 0, st>>>(A);
-        MTB_CHECK_LAUNCH();
+        if ((rc = go(fe[mode + (fin ? 4 : 0)], grid, blk, A, en, eo, rec_comp_stride))) return rc;
+        if ((rc = go(k_adj3_h, grid, blk, A))) return rc;
         p->last_launches += 2;
         if (q > 0 && (rc = inject(q - 1))) return rc;    // before the fin + E launch of q - 1
     }
-    k_adj3_fin<<<grid, blk, 0, st>>>(A);
-    MTB_CHECK_LAUNCH();
-    k_adj3_eps<<<grid, A3_T, 0, st>>>(A);
-    MTB_CHECK_LAUNCH();
+    if ((rc = go(k_adj3_fin, grid, blk, A)) || (rc = go(k_adj3_eps, grid, A3_T, A))) return rc;
     p->last_launches += 2;
     return MTB_OK;
 }

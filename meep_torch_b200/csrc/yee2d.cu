@@ -1787,7 +1787,9 @@ __global__ void __launch_bounds__(32 * TROWS, 2) k_tile_tm(
     Ctx2D C) {
     __shared__ TileSmem T;
     int4 w;
+    pdl_next();
     if (!tile_setup(SS, work, n_work, C.wr, T, w)) return;
+    pdl_wait();                 // tile list, descriptors and lines are constant
     const mtb_yee2d_struct &S = T.s;
     const int ib = w.y + threadIdx.y * C.wr;           // this warp's rows ib .. ib+wr-1
     if (ib >= S.nx) return;                             // whole warp
@@ -2020,7 +2022,9 @@ __global__ void __launch_bounds__(32 * TROWS, 2) k_tile_te(
     Ctx2D C) {
     __shared__ TileSmem T;
     int4 w;
+    pdl_next();
     if (!tile_setup(SS, work, n_work, C.wr, T, w)) return;
+    pdl_wait();                 // tile list, descriptors and lines are constant
     const mtb_yee2d_struct &S = T.s;
     const int ib = w.y + threadIdx.y * C.wr;
     if (ib >= S.nx) return;
@@ -2754,33 +2758,34 @@ static int launch_step(mtb_yee2d_plan *p, const Ctx2D &C, cudaStream_t st) {
     const int n_tm = p->n_work_tm, n_te = p->n_work - p->n_work_tm;
     const mtb_yee2d_struct *SS = p->structs_d.as<mtb_yee2d_struct>();
     const int4 *W = p->work_d.as<int4>();
+    int rc = MTB_OK;
     if (p->variant == 2) {
         const dim3 blk(32, TROWS);
         if (n_tm > 0) {
             if (p->mpoles) {
                 // magnetic Lorentz poles: their own instantiation (more live registers)
                 if (C.first)
-                    k_tile_tm<true, true, true><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
+                    rc = launch_pdl(k_tile_tm<true, true, true>, n_tm, blk, st, SS, W, n_tm, C);
                 else
-                    k_tile_tm<false, true, true><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
+                    rc = launch_pdl(k_tile_tm<false, true, true>, n_tm, blk, st, SS, W, n_tm, C);
             } else if (C.first && p->ext)
-                k_tile_tm<true, true><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
+                rc = launch_pdl(k_tile_tm<true, true>, n_tm, blk, st, SS, W, n_tm, C);
             else if (C.first)
-                k_tile_tm<true, false><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
+                rc = launch_pdl(k_tile_tm<true, false>, n_tm, blk, st, SS, W, n_tm, C);
             else if (p->ext)
-                k_tile_tm<false, true><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
+                rc = launch_pdl(k_tile_tm<false, true>, n_tm, blk, st, SS, W, n_tm, C);
             else
-                k_tile_tm<false, false><<<n_tm, blk, 0, st>>>(SS, W, n_tm, C);
-            MTB_CHECK_LAUNCH();
+                rc = launch_pdl(k_tile_tm<false, false>, n_tm, blk, st, SS, W, n_tm, C);
+            if (rc) return rc;
             ++p->last_launches;
         }
         const int n_t3 = p->n_work_te3, n_te1 = n_te - n_t3;
         if (n_te1 > 0) {
             if (p->ext)
-                k_tile_te<true><<<n_te1, blk, 0, st>>>(SS, W + n_tm, n_te1, C);
+                rc = launch_pdl(k_tile_te<true>, n_te1, blk, st, SS, W + n_tm, n_te1, C);
             else
-                k_tile_te<false><<<n_te1, blk, 0, st>>>(SS, W + n_tm, n_te1, C);
-            MTB_CHECK_LAUNCH();
+                rc = launch_pdl(k_tile_te<false>, n_te1, blk, st, SS, W + n_tm, n_te1, C);
+            if (rc) return rc;
             ++p->last_launches;
         }
         if (n_t3 > 0) {

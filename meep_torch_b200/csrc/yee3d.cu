@@ -582,17 +582,17 @@ __device__ __forceinline__ void s3_h(const Split3 &P, const S3Cell &c) {
     z4(fa); z4(fan); z4(fb); z4(fbn); z4(h); z4(pa); z4(pb);
     float zk = 0.f;                                       // E(k+1) of q = 3
     if (act) {
-        ldg4v(P.e[FA] + g, fa);
-        ldg4v(P.e[FB] + g, fb);
-        if (AA == 1 && j + 1 < ny) ldg4v(P.e[FA] + g + ZP, fan);
-        if (AA == 0 && i + 1 < nx) ldg4v(P.e[FA] + g + NYZ, fan);
-        if (AB == 1 && j + 1 < ny) ldg4v(P.e[FB] + g + ZP, fbn);
-        if (AB == 0 && i + 1 < nx) ldg4v(P.e[FB] + g + NYZ, fbn);
+        ld4v(P.e[FA] + g, fa);
+        ld4v(P.e[FB] + g, fb);
+        if (AA == 1 && j + 1 < ny) ld4v(P.e[FA] + g + ZP, fan);
+        if (AA == 0 && i + 1 < nx) ld4v(P.e[FA] + g + NYZ, fan);
+        if (AB == 1 && j + 1 < ny) ld4v(P.e[FB] + g + ZP, fbn);
+        if (AB == 0 && i + 1 < nx) ld4v(P.e[FB] + g + NYZ, fbn);
         if (C != 2 && (threadIdx.x & 31) == 31 && kb + 4 < ZP)
-            zk = __ldg(P.e[AA == 2 ? FA : FB] + g + 4);
-        ldg4v(P.h[C] + g, h);
-        if (pa_on) ldg4v(P.pi[2 * C] + g, pa);
-        if (pb_on) ldg4v(P.pi[2 * C + 1] + g, pb);
+            zk = P.e[AA == 2 ? FA : FB][g + 4];
+        ld4v(P.h[C] + g, h);
+        if (pa_on) ld4v(P.pi[2 * C] + g, pa);
+        if (pb_on) ld4v(P.pi[2 * C + 1] + g, pb);
     }
     float a1[4], a2[4];
     if (DAMP && act) {
@@ -633,7 +633,9 @@ __device__ __forceinline__ void s3_h(const Split3 &P, const S3Cell &c) {
 
 template <bool DAMP>
 __global__ void __launch_bounds__(3 * S3_T, 3) k_yee3d_h(const __grid_constant__ Split3 P, int i0) {
+    pdl_next();
     const S3Cell c(P, i0 + blockIdx.y);
+    pdl_wait();
     if (threadIdx.y == 0) s3_h<0, DAMP>(P, c);
     else if (threadIdx.y == 1) s3_h<1, DAMP>(P, c);
     else s3_h<2, DAMP>(P, c);
@@ -681,20 +683,20 @@ __device__ __forceinline__ void s3_e(const Split3 &P, const S3Cell &c,
     int e0 = 0, e1x = 0;                                  // soft current cells of row (i, j)
     float pc[4], pq[4], c3[4];                            // first pole: P(n), P(n-1), drive
     if (act) {
-        ldg4v(Ha + g, ha);
-        ldg4v(Hb + g, hb);
+        ld4v(Ha + g, ha);
+        ld4v(Hb + g, hb);
         ldg4v(P.eps + g, ep);
-        ldg4v(P.e[C] + g, en);
-        if (AA == 1 && j >= 1) ldg4v(Ha + g - ZP, hap);
-        if (AA == 0 && i >= 1) ldg4v(Ha + g - NYZ, hap);
-        if (AB == 1 && j >= 1) ldg4v(Hb + g - ZP, hbp);
-        if (AB == 0 && i >= 1) ldg4v(Hb + g - NYZ, hbp);
+        ld4v(P.e[C] + g, en);
+        if (AA == 1 && j >= 1) ld4v(Ha + g - ZP, hap);
+        if (AA == 0 && i >= 1) ld4v(Ha + g - NYZ, hap);
+        if (AB == 1 && j >= 1) ld4v(Hb + g - ZP, hbp);
+        if (AB == 0 && i >= 1) ld4v(Hb + g - NYZ, hbp);
         if (C == 0 && i + 1 < nx) ldg4v(P.eps + g + NYZ, epn);
         if (C == 1 && j + 1 < ny) ldg4v(P.eps + g + ZP, epn);
         if (C == 2 && lane == 31 && kb + 4 < ZP) epk = __ldg(P.eps + g + 4);
-        if (C != 2 && lane == 0 && kb >= 1) zk = __ldg((AA == 2 ? Ha : Hb) + g - 1);
-        if (pa_on) ldg4v(P.pi[6 + 2 * C] + g, pa);
-        if (pb_on) ldg4v(P.pi[7 + 2 * C] + g, pb);
+        if (C != 2 && lane == 0 && kb >= 1) zk = (AA == 2 ? Ha : Hb)[g - 1];
+        if (pa_on) ld4v(P.pi[6 + 2 * C] + g, pa);
+        if (pb_on) ld4v(P.pi[7 + 2 * C] + g, pb);
         if (PL) {
             ld4v(P.pp[C][0] + g, pc);
             ld4v(P.pp[C][1] + g, pq);
@@ -795,7 +797,9 @@ __device__ __forceinline__ void s3_e(const Split3 &P, const S3Cell &c,
 template <int MODE>                 // bit 0: damping, bit 1: poles
 __global__ void __launch_bounds__(3 * S3_T, MODE ? 2 : 3)
 k_yee3d_e(const __grid_constant__ Split3 P, const float *__restrict__ amp, int i0) {
+    pdl_next();
     const S3Cell c(P, i0 + blockIdx.y);
+    pdl_wait();
     if (threadIdx.y == 0) s3_e<0, MODE>(P, c, amp);
     else if (threadIdx.y == 1) s3_e<1, MODE>(P, c, amp);
     else s3_e<2, MODE>(P, c, amp);
@@ -806,7 +810,11 @@ __global__ void k_sample3d(const mtb_yee3d_struct *__restrict__ SS, const int64_
                            int n_planes, int cur, float *__restrict__ ring) {
     const mtb_yee3d_struct &S = *SS;
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= pstart[n_planes]) return;
+    pdl_next();
+    if (e >= pstart[n_planes]) {
+        pdl_wait();
+        return;
+    }
     int lo = 0, hi = n_planes - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
@@ -822,6 +830,7 @@ __global__ void k_sample3d(const mtb_yee3d_struct *__restrict__ SS, const int64_
     else if (axis == 1) { i = a; j = index; k = b; }
     else { i = a; j = b; k = index; }
     const float *F = S.f[comp][cur];
+    pdl_wait();                          // the descriptor and plane tables are constant
     ring[S.plane_ring_off[lo] + p] = F[((int64_t)i * S.ny + j) * S.zpitch + k];
 }
 
@@ -1397,21 +1406,22 @@ static int launch_split(mtb_yee3d_plan *p, const Split3 &sp, int part, int i0, i
     if (i1 <= i0) return MTB_OK;
     const dim3 grid((unsigned)(((int64_t)p->s.ny * (p->s.zpitch / 4) + S3_T - 1) / S3_T), i1 - i0);
     const dim3 block(S3_T, 3);
+    int rc;
     if (part == 0) {
         if (p->damp)
-            k_yee3d_h<true><<<grid, block, 0, st>>>(sp, i0);
+            rc = launch_pdl(k_yee3d_h<true>, grid, block, st, sp, i0);
         else
-            k_yee3d_h<false><<<grid, block, 0, st>>>(sp, i0);
+            rc = launch_pdl(k_yee3d_h<false>, grid, block, st, sp, i0);
     } else {
         const float *a = p->amp_d.as<float>() + s;
         switch ((p->damp ? 1 : 0) | (p->poles ? 2 : 0)) {
-            case 0: k_yee3d_e<0><<<grid, block, 0, st>>>(sp, a, i0); break;
-            case 1: k_yee3d_e<1><<<grid, block, 0, st>>>(sp, a, i0); break;
-            case 2: k_yee3d_e<2><<<grid, block, 0, st>>>(sp, a, i0); break;
-            default: k_yee3d_e<3><<<grid, block, 0, st>>>(sp, a, i0); break;
+            case 0: rc = launch_pdl(k_yee3d_e<0>, grid, block, st, sp, a, i0); break;
+            case 1: rc = launch_pdl(k_yee3d_e<1>, grid, block, st, sp, a, i0); break;
+            case 2: rc = launch_pdl(k_yee3d_e<2>, grid, block, st, sp, a, i0); break;
+            default: rc = launch_pdl(k_yee3d_e<3>, grid, block, st, sp, a, i0); break;
         }
     }
-    MTB_CHECK_LAUNCH();
+    if (rc) return rc;
     ++p->last_launches;
     return MTB_OK;
 }
@@ -1425,10 +1435,9 @@ static int finish_step(mtb_yee3d_plan *p, cudaStream_t st) {
     if (sampling) {
         float *ring = p->dft.ring_d.as<float>() + (size_t)p->c_slot * p->dft.slot_elems;
         const int64_t nb = (p->n_samples + 255) / 256;
-        k_sample3d<<<(unsigned)nb, 256, 0, st>>>(p->s_d.as<mtb_yee3d_struct>(),
-                                                p->pstart_d.as<int64_t>(), p->n_planes, p->par,
-                                                ring);
-        MTB_CHECK_LAUNCH();
+        if ((rc = launch_pdl(k_sample3d, (unsigned)nb, 256, st, p->s_d.as<mtb_yee3d_struct>(),
+                             p->pstart_d.as<int64_t>(), p->n_planes, p->par, ring)))
+            return rc;
         ++p->last_launches;
     }
     const int s = p->c_s;
