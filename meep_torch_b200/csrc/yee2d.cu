@@ -207,6 +207,21 @@ __device__ __forceinline__ void apply_cells(const mtb_cells &cl, int row, const 
             if (c == q) v[q] -= a * w;
     }
 }
+// the same with the rounding spelled out: product, then difference
+__device__ __forceinline__ void apply_cells_rn(const mtb_cells &cl, int row, const float *amp,
+                                               int jb, float (&v)[4]) {
+    const int e0 = __ldg(cl.row_ptr + row), e1 = __ldg(cl.row_ptr + row + 1);
+    if (e0 == e1) return;
+    const float a = __ldg(amp + cl.amp_col);
+    for (int e = lower_col(cl.col, e0, e1, jb); e < e1; ++e) {
+        const int c = __ldg(cl.col + e) - jb;
+        if (c >= 4) break;
+        const float aw = __fmul_rn(a, __ldg(cl.w + e));
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (c == q) v[q] = __fsub_rn(v[q], aw);
+    }
+}
 __device__ __forceinline__ float apply_cell1(const mtb_cells &cl, int row, int col,
                                              const float *amp, float v) {
     if (cl.n == 0 || row < cl.row_lo || row > cl.row_hi) return v;
@@ -2172,6 +2187,48 @@ static int d2h_floats(std::vector<float> &h, const float *d, int n, int s) {
 // structure's padded profiles are 4 y rows (hy b, a; ey b, a) of pitch + 128
 // floats, column j at index j + 4, then 4 x rows (hx b, a; ex b, a) of
 // nx + 32 floats, row i at index i + 4; inert (1, 0) off the arrays.
+// Orders n tiles (work items from `first`) so that the blocks' shares cost the same: block b
+// of a grid of g takes tiles b, b + g, b + 2g, ... In the order of rows and columns a share
+// is one column of tiles whenever g is a multiple of the tiles per row, and a tile that
+// reaches a y layer costs 1.8 (TM) to 2.1 (TE) times a lean one: the last of 148 blocks ended
+// after 65 us where the mean ended after 44 us (12 structures of 480 x 480; with the balance a
+// launch takes 52 us in place of 66). Each wave of g
+// tiles keeps its tiles (neighbours share their halos through L2); within a wave the costliest
+// tile goes to the block with the least so far. The last, partial wave is the blocks' first g'
+// by construction, so it is counted first.
+static void tb_balance(std::vector<int4> &work, int first, int n, int g) {
+    struct Tile { int cost; int4 rec[TB_WORK]; };
+    if (n <= g) return;
+    std::vector<int64_t> load(g, 0);
+    std::vector<int> order(g);
+    std::vector<Tile> tiles;
+    auto wave = [&](int w0, int m) {
+        tiles.resize(m);
+        for (int t = 0; t < m; ++t) {
+            const int4 *r = work.data() + (size_t)TB_WORK * (first + w0 + t);
+            const int f = r[0].w;
+            const bool y = ((f >> TBF_YSHIFT) & 3) != TBF_YNONE;
+            tiles[t].cost = (f & TBF_LEAN) ? 10 : y ? 19 : 14;
+            std::copy(r, r + TB_WORK, tiles[t].rec);
+        }
+        std::stable_sort(tiles.begin(), tiles.end(),
+                         [](const Tile &a, const Tile &b) { return a.cost > b.cost; });
+        order.resize(m);
+        for (int b = 0; b < m; ++b) order[b] = b;
+        std::stable_sort(order.begin(), order.end(),
+                         [&](int a, int b) { return load[a] < load[b]; });
+        for (int t = 0; t < m; ++t) {
+            const int b = order[t];
+            load[b] += tiles[t].cost;
+            std::copy(tiles[t].rec, tiles[t].rec + TB_WORK,
+                      work.begin() + (size_t)TB_WORK * (first + w0 + b));
+        }
+    };
+    const int full = n / g * g;
+    if (full < n) wave(full, n - full);
+    for (int w0 = 0; w0 < full; w0 += g) wave(w0, g);
+}
+
 static int tb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs) {
     const int n = (int)structs.size();
     std::vector<CUtensorMap> maps((size_t)n * TBM_N);
@@ -2292,6 +2349,12 @@ static int tb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> 
         if (pol == 0) p->n_tb_tm = (int)(work.size() / TB_WORK);
     }
     p->n_tb_te = (int)(work.size() / TB_WORK) - p->n_tb_tm;
+    int dev = 0, sms = 0;
+    MTB_CUDA_TRY(cudaGetDevice(&dev));
+    MTB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    p->tb_grid = std::max(sms, 1);
+    tb_balance(work, 0, p->n_tb_tm, p->tb_grid);
+    tb_balance(work, p->n_tb_tm, p->n_tb_te, p->tb_grid);
     if ((rc = p->tmaps_d.ensure(sizeof(CUtensorMap) * maps.size())) ||
         (rc = p->tb_work_d.ensure(sizeof(int4) * std::max<size_t>(work.size(), 1))) ||
         (rc = p->tb_meta_d.ensure(sizeof(TbMeta) * metas.size())) ||
@@ -2314,11 +2377,7 @@ static int tb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> 
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_tb_te, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)tb_smem<true>());
-    int dev = 0, sms = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return fail(MTB_CUDA_ERROR, "TB set-up: %s", cudaGetErrorString(e));
-    p->tb_grid = std::max(sms, 1);
     p->tb = true;
     return MTB_OK;
 }

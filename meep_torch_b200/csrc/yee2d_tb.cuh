@@ -13,12 +13,20 @@
 // aligned.
 //
 // Block. One 1024-thread block per SM, persistent over a static share of the
-// tiles: warp w owns tile row w, lane L columns 4L .. 4L+3. A thread keeps its
+// tiles (balanced by cost): warp w owns tile row w, lane L columns 4L .. 4L+3. A thread keeps its
 // cells' fields, 1/eps and x-layer CPML memory in registers for all sub-steps;
 // the y-layer CPML memory (only lanes with a y-layer column touch it) stays in
 // shared memory. Rows exchange through two shared-memory planes (TM: Ez for
 // the row above's Hy update, Hy for the row below's Dz update; TE: Hz and Ey),
-// two barriers per sub-step; columns exchange through warp shuffles.
+// two barriers per sub-step; columns exchange through warp shuffles. A lean TM
+// tile (no layer, no wall) updates the neighbour's Hy row too and needs one.
+//
+// What bounds it: instruction issue, 2-3 us per tile for taking, set-up and
+// storing and 1.0-1.4 us per sub-step (TM lean; 480 x 480). Per launch of 4
+// steps: 10 TM structures of about 512 x 512 78 -> 69 us, TE 90 -> 78 us, 64 TM
+// of 256 x 256 156 -> 153 us (all its tiles reach a y layer). The barriers
+// themselves cost little; registers do: 64 a thread, and each form below that
+// spilled more lost more than it saved.
 //
 // Staging. Everything a tile reads is brought into shared memory by the bulk
 // copy engine, completion counted on one mbarrier: the field, 1/eps and CPML
@@ -37,6 +45,8 @@
 // par ^ 1, whatever its sub-step count. Monitor samples of every sub-step go
 // to consecutive ring slots, written by the thread owning the output cell.
 #include <cuda.h>
+
+#include <type_traits>
 
 namespace mtb {
 
@@ -96,7 +106,6 @@ struct TbCtl {
     int4 rec[2][3];          // tile records, by tile parity (read ahead one tile)
     int4 cur[2];             // work item a of the tiles held in buffer sets 0, 1
     uint64_t bar;
-    int ok;
 };
 
 template <bool TE>
@@ -198,14 +207,15 @@ __device__ __forceinline__ void tb_issue(const CUtensorMap *__restrict__ maps, c
     }
 }
 
-// Thread 0 waits (bounded) for tile k's copies; block-uniform verdict in ctl->ok.
-__device__ __forceinline__ void tb_wait(TbCtl &ctl, uint32_t parity, int *err) {
+// Bounded wait of each thread for tile k's copies (which also acquires them). False if it
+// expired; the caller's next barrier makes that block-uniform.
+__device__ __forceinline__ bool tb_wait(TbCtl &ctl, uint32_t parity, int *err) {
     bool ok = mbar_try_wait(&ctl.bar, parity);
     if (!ok) {
         const unsigned long long t0 = gtimer();
         while (!(ok = mbar_try_wait(&ctl.bar, parity)) && gtimer() - t0 < WAIT_NS) {
         }
-        if (!ok) {
+        if (!ok && threadIdx.x == 0) {
             atomicExch(err, 1);
             // let the copies in flight land before the block exits (bounded)
             const unsigned long long t1 = gtimer();
@@ -213,7 +223,7 @@ __device__ __forceinline__ void tb_wait(TbCtl &ctl, uint32_t parity, int *err) {
             }
         }
     }
-    ctl.ok = ok ? 1 : 0;
+    return ok;
 }
 
 // Copy a staged float4 (plane a, this thread's cells) to registers.
@@ -250,6 +260,16 @@ __device__ __forceinline__ void tb_take_psi(const float *ps, int flags, int w, i
     }
 }
 
+// (a - b) / dx; the CPML term d + q with q = b psi + a d (kappa = 1), psi <- q. Rounding is
+// spelled out here and in the sub-steps: all 2D kernels give a plan the same bits.
+__device__ __forceinline__ float tb_d(float a, float b, float rdx) {
+    return __fmul_rn(__fsub_rn(a, b), rdx);
+}
+__device__ __forceinline__ float tb_cpml(float d, float b, float a, float &psi) {
+    psi = __fmaf_rn(b, psi, __fmul_rn(a, d));
+    return __fadd_rn(d, psi);
+}
+
 // Copy this row's values of component `comp` into the line samples of `mask`.
 __device__ __forceinline__ void tb_sample(const mtb_line_sample *L, unsigned mask, int comp,
                                           int i, int jb, const float (&v)[4], float *ring) {
@@ -275,17 +295,6 @@ __device__ __forceinline__ void tb_sample(const mtb_line_sample *L, unsigned mas
     }
 }
 
-// Tile start, common to TM and TE: thread 0's bounded wait for tile k's copies,
-// the block-uniform verdict, and each thread's acquire of the completed phase.
-template <bool TE>
-__device__ __forceinline__ bool tb_begin(uint32_t k, TbLayout<TE> &L, int *err) {
-    if (threadIdx.x == 0) tb_wait(*L.ctl, k & 1, err);
-    __syncthreads();
-    if (!L.ctl->ok) return false;
-    (void)mbar_try_wait(&L.ctl->bar, k & 1);     // completed: acquire for this thread
-    return true;
-}
-
 // Block start, common to TM and TE: barrier init and the first tile's copies
 // (with the second tile's record).
 template <bool TE>
@@ -299,6 +308,7 @@ __device__ __forceinline__ void tb_start(const CUtensorMap *__restrict__ maps, c
         tb_issue<TE>(maps, C, __ldg(r), __ldg(r + 1), __ldg(r + 2), work,
                      blockIdx.x + gridDim.x, n_work, L, 0);
     }
+    __syncthreads();                                // the barrier is initialised
 }
 
 // After tile k's planes are taken: thread 0 issues tile k+1's copies from its
@@ -330,7 +340,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
     const int par = C.par, pn = par ^ 1;
     const int cell = w * TB_C + 4 * lane;             // this thread's offset in a plane
     for (uint32_t k = 0; it < n_work; ++k, it += gridDim.x) {
-        if (!tb_begin<false>(k, L, C.err)) return;
+        const bool ok = tb_wait(*L.ctl, k & 1, C.err);
         const int4 wk = L.ctl->cur[k & 1];
         const TbMeta &M = L.meta[k & 1];
         const mtb_yee2d_struct &S = M.s;
@@ -339,8 +349,12 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
         tb_take(L.stage, 1, cell, hx);
         tb_take(L.stage, 2, cell, hy);
         tb_take(L.stage, 3, cell, ie);
-        tb_take_psi(L.stage + NF * TB_PLANE, wk.w, w, lane, p1, p2, L.yp);
-        __syncthreads();                                // staging planes are free
+        const bool lean = wk.w & TBF_LEAN;
+        if (lean)                                       // p1: Hy of the row above
+            tb_take(L.stage, 2, w > 0 ? cell - TB_C : cell, p1);
+        else
+            tb_take_psi(L.stage + NF * TB_PLANE, wk.w, w, lane, p1, p2, L.yp);
+        if (!__syncthreads_and(ok)) return;             // staging planes are free
         tb_next<false>(maps, C, work, n_work, it, k, L);
 
         const int nx = S.nx, ny = S.ny, P = S.pitch;
@@ -350,6 +364,80 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
         const bool rowIn = i >= 0 && i < nx;
         const bool hyRow = i >= 0 && i <= nx - 2, dzRow = i >= 1 && i <= nx - 2;
         const float dt = S.dt, rdx = 1.0f / S.dx;
+        const bool outC = act && lane >= 1 && lane <= 30;
+        const bool out = outC && rowIn && w >= TB_T && w < TB_T + TB_OUTR;
+        const unsigned lmask = (unsigned)wk.w >> TBF_LINE_SHIFT;
+        const uint32_t ro = (uint32_t)(i * P + jb);
+        const bool srcE = act && rowIn && S.src_e.n > 0 && i >= S.src_e.row_lo &&
+                          i <= S.src_e.row_hi;
+        const bool srcH1 = act && hyRow && S.src_h1.n > 0 && i >= S.src_h1.row_lo &&
+                           i <= S.src_h1.row_hi;
+        const bool srcH2 = act && rowIn && S.src_h2.n > 0 && i >= S.src_h2.row_lo &&
+                           i <= S.src_h2.row_hi;
+        if (lean) {
+            // every cell of the tile is updated and no CPML term is active: no validity
+            // masks or CPML memory, and one barrier a sub-step. The Ez rows alternate between
+            // the two exchange planes, and each warp also updates the Hy row above its own
+            // (hya), which Dz reads. Rounding is spelled out: that of the other tiles.
+            float *rs0 = (out && S.ring_full[0] >= 0) ? C.ring + S.ring_full[0] + ro : nullptr;
+            float *rs1 = (out && S.ring_full[1] >= 0) ? C.ring + S.ring_full[1] + ro : nullptr;
+            float *rs2 = (out && S.ring_full[2] >= 0) ? C.ring + S.ring_full[2] + ro : nullptr;
+            const bool srcH1a = act && S.src_h1.n > 0 && i > S.src_h1.row_lo &&
+                                i <= S.src_h1.row_hi + 1;
+            const int above = w > 0 ? -TB_C : 0, below = w + 1 < TB_R ? TB_C : 0;
+            float(&hya)[4] = p1;
+            float ez[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) ez[q] = __fmul_rn(dz[q], ie[q]);
+            for (int s = 0; s < C.nsub; ++s) {
+                float *x = ((s & 1) ? xh : xe) + cell;
+                st4(x, ez);
+                __syncthreads();
+                float ea[4], eb[4];
+                lds4(x + above, ea);
+                lds4(x + below, eb);
+                const float ezR = __shfl_down_sync(0xffffffffu, ez[0], 1);
+                const float *ah = C.amp_h + s * C.ncols;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float er = (q < 3) ? ez[q + 1] : ezR;
+                    hx[q] = __fmaf_rn(-dt, __fmul_rn(__fsub_rn(er, ez[q]), rdx), hx[q]);
+                    hy[q] = __fmaf_rn(dt, __fmul_rn(__fsub_rn(eb[q], ez[q]), rdx), hy[q]);
+                    hya[q] = __fmaf_rn(dt, __fmul_rn(__fsub_rn(ez[q], ea[q]), rdx), hya[q]);
+                }
+                if (srcH2) apply_cells_rn(S.src_h2, i, ah, jb, hx);
+                if (srcH1) apply_cells_rn(S.src_h1, i, ah, jb, hy);
+                if (srcH1a) apply_cells_rn(S.src_h1, i - 1, ah, jb, hya);
+                const float hxm0 = __shfl_up_sync(0xffffffffu, hx[3], 1);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float hxm = (q == 0) ? hxm0 : hx[q - 1];
+                    const float dhx = __fmul_rn(__fsub_rn(hx[q], hxm), rdx);
+                    dz[q] = __fmaf_rn(dt, __fmaf_rn(__fsub_rn(hy[q], hya[q]), rdx, -dhx), dz[q]);
+                }
+                if (srcE) apply_cells_rn(S.src_e, i, C.amp_e + s * C.ncols, jb, dz);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ez[q] = __fmul_rn(dz[q], ie[q]);
+                if (out) {
+                    const int64_t so = s * C.slot_elems;
+                    if (rs0) st4(rs0 + so, ez);
+                    if (rs1) st4(rs1 + so, hx);
+                    if (rs2) st4(rs2 + so, hy);
+                    if (lmask) {
+                        float *ring = C.ring + so;
+                        tb_sample(M.lines, lmask, MTB_C2_MAIN, i, jb, ez, ring);
+                        tb_sample(M.lines, lmask, MTB_C2_X, i, jb, hx, ring);
+                        tb_sample(M.lines, lmask, MTB_C2_Y, i, jb, hy, ring);
+                    }
+                }
+            }
+            if (out) {
+                st4(S.f_main[pn] + ro, dz);
+                st4(S.f_x[pn] + ro, hx);
+                st4(S.f_y[pn] + ro, hy);
+            }
+            continue;
+        }
         unsigned mHx = 0, mHy = 0, mD = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -371,76 +459,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
         const bool yl = ((wk.w >> TBF_YSHIFT) & 3) != TBF_YNONE;
         float *yp0 = L.yp + cell, *yp3 = L.yp + TB_PLANE + cell;
         const float *pr = L.prof + (k & 1) * 4 * TB_C + 4 * lane;
-        const bool outC = act && lane >= 1 && lane <= 30;
-        const bool out = outC && rowIn && w >= TB_T && w < TB_T + TB_OUTR;
-        const unsigned lmask = (unsigned)wk.w >> TBF_LINE_SHIFT;
-        const uint32_t ro = (uint32_t)(i * P + jb);
-        const bool srcE = act && rowIn && S.src_e.n > 0 && i >= S.src_e.row_lo &&
-                          i <= S.src_e.row_hi;
-        const bool srcH1 = act && hyRow && S.src_h1.n > 0 && i >= S.src_h1.row_lo &&
-                           i <= S.src_h1.row_hi;
-        const bool srcH2 = act && rowIn && S.src_h2.n > 0 && i >= S.src_h2.row_lo &&
-                           i <= S.src_h2.row_hi;
-        if (wk.w & TBF_LEAN) {
-            // every cell of the tile is updated and no CPML term is active: the
-            // same arithmetic without validity masks or CPML memory
-            float *rs0 = (out && S.ring_full[0] >= 0) ? C.ring + S.ring_full[0] + ro : nullptr;
-            float *rs1 = (out && S.ring_full[1] >= 0) ? C.ring + S.ring_full[1] + ro : nullptr;
-            float *rs2 = (out && S.ring_full[2] >= 0) ? C.ring + S.ring_full[2] + ro : nullptr;
-            for (int s = 0; s < C.nsub; ++s) {
-                float ez[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) ez[q] = dz[q] * ie[q];
-                st4(xe + cell, ez);
-                __syncthreads();
-                float eb[4];
-                if (w + 1 < TB_R) lds4(xe + cell + TB_C, eb);
-                else zero4(eb);
-                const float ezR = __shfl_down_sync(0xffffffffu, ez[0], 1);
-                const float *ah = C.amp_h + s * C.ncols;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float er = (q < 3) ? ez[q + 1] : ezR;
-                    hx[q] = hx[q] - dt * ((er - ez[q]) * rdx);
-                    hy[q] = hy[q] + dt * ((eb[q] - ez[q]) * rdx);
-                }
-                if (srcH2) apply_cells(S.src_h2, i, ah, jb, hx);
-                if (srcH1) apply_cells(S.src_h1, i, ah, jb, hy);
-                st4(xh + cell, hy);
-                __syncthreads();
-                float ha[4];
-                if (w > 0) lds4(xh + cell - TB_C, ha);
-                else zero4(ha);
-                const float hxm0 = __shfl_up_sync(0xffffffffu, hx[3], 1);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float hxm = (q == 0) ? hxm0 : hx[q - 1];
-                    const float dhy = (hy[q] - ha[q]) * rdx;
-                    const float dhx = (hx[q] - hxm) * rdx;
-                    dz[q] = dz[q] + dt * (dhy - dhx);
-                }
-                if (srcE) apply_cells(S.src_e, i, C.amp_e + s * C.ncols, jb, dz);
-                if (out) {
-                    float ezN[4];
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) ezN[q] = dz[q] * ie[q];
-                    const int64_t so = s * C.slot_elems;
-                    if (rs0) st4(rs0 + so, ezN);
-                    if (rs1) st4(rs1 + so, hx);
-                    if (rs2) st4(rs2 + so, hy);
-                    if (lmask) {
-                        float *ring = C.ring + so;
-                        tb_sample(M.lines, lmask, MTB_C2_MAIN, i, jb, ezN, ring);
-                        tb_sample(M.lines, lmask, MTB_C2_X, i, jb, hx, ring);
-                        tb_sample(M.lines, lmask, MTB_C2_Y, i, jb, hy, ring);
-                    }
-                }
-            }
-        } else
         for (int s = 0; s < C.nsub; ++s) {
             float ez[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) ez[q] = dz[q] * ie[q];
+            for (int q = 0; q < 4; ++q) ez[q] = __fmul_rn(dz[q], ie[q]);
             st4(xe + cell, ez);
             __syncthreads();
             float eb[4];
@@ -457,9 +479,9 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float er = (q < 3) ? ez[q + 1] : ezR;
-                    const float d = (er - ez[q]) * rdx;
-                    const float pv = b[q] * p0[q] + a[q] * d;
-                    const float hn = hx[q] - dt * (d + pv);
+                    float pv = p0[q];
+                    const float c = tb_cpml(tb_d(er, ez[q], rdx), b[q], a[q], pv);
+                    const float hn = __fmaf_rn(-dt, c, hx[q]);
                     const bool v = (mHx >> q) & 1u;
                     hx[q] = v ? hn : hx[q];
                     p0[q] = v ? pv : p0[q];
@@ -469,18 +491,18 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float er = (q < 3) ? ez[q + 1] : ezR;
-                    const float hn = hx[q] - dt * ((er - ez[q]) * rdx);
+                    const float hn = __fmaf_rn(-dt, tb_d(er, ez[q], rdx), hx[q]);
                     hx[q] = ((mHx >> q) & 1u) ? hn : hx[q];
                 }
             }
-            if (srcH2) apply_cells(S.src_h2, i, ah, jb, hx);
+            if (srcH2) apply_cells_rn(S.src_h2, i, ah, jb, hx);
             // Hy(n+1/2)
             if (bxH) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float d = (eb[q] - ez[q]) * rdx;
-                    const float pv = hxb * p1[q] + hxa * d;
-                    const float hn = hy[q] + dt * (d + pv);
+                    float pv = p1[q];
+                    const float c = tb_cpml(tb_d(eb[q], ez[q], rdx), hxb, hxa, pv);
+                    const float hn = __fmaf_rn(dt, c, hy[q]);
                     const bool v = (mHy >> q) & 1u;
                     hy[q] = v ? hn : hy[q];
                     p1[q] = v ? pv : p1[q];
@@ -488,11 +510,11 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float hn = hy[q] + dt * ((eb[q] - ez[q]) * rdx);
+                    const float hn = __fmaf_rn(dt, tb_d(eb[q], ez[q], rdx), hy[q]);
                     hy[q] = ((mHy >> q) & 1u) ? hn : hy[q];
                 }
             }
-            if (srcH1) apply_cells(S.src_h1, i, ah, jb, hy);
+            if (srcH1) apply_cells_rn(S.src_h1, i, ah, jb, hy);
             st4(xh + cell, hy);
             __syncthreads();
             float ha[4];
@@ -513,12 +535,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float hxm = (q == 0) ? hxm0 : hx[q - 1];
-                    const float dhy = (hy[q] - ha[q]) * rdx;
-                    const float dhx = (hx[q] - hxm) * rdx;
-                    const float q2 = exb * p2[q] + exa * dhy;
-                    const float q3 = b3[q] * p3[q] + a3[q] * dhx;
-                    const float curl = (dhy + q2) - (dhx + q3);
-                    const float dn = dz[q] + dt * curl;
+                    float q2 = p2[q], q3 = p3[q];
+                    const float ty = tb_cpml(tb_d(hy[q], ha[q], rdx), exb, exa, q2);
+                    const float tx = tb_cpml(tb_d(hx[q], hxm, rdx), b3[q], a3[q], q3);
+                    const float dn = __fmaf_rn(dt, __fsub_rn(ty, tx), dz[q]);
                     const bool v = (mD >> q) & 1u;
                     dz[q] = v ? dn : dz[q];
                     p2[q] = v ? q2 : p2[q];
@@ -529,17 +549,17 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float hxm = (q == 0) ? hxm0 : hx[q - 1];
-                    const float dhy = (hy[q] - ha[q]) * rdx;
-                    const float dhx = (hx[q] - hxm) * rdx;
-                    const float dn = dz[q] + dt * (dhy - dhx);
+                    const float dhx = tb_d(hx[q], hxm, rdx);
+                    const float dn = __fmaf_rn(dt, __fmaf_rn(__fsub_rn(hy[q], ha[q]), rdx, -dhx),
+                                               dz[q]);
                     dz[q] = ((mD >> q) & 1u) ? dn : dz[q];
                 }
             }
-            if (srcE) apply_cells(S.src_e, i, C.amp_e + s * C.ncols, jb, dz);
+            if (srcE) apply_cells_rn(S.src_e, i, C.amp_e + s * C.ncols, jb, dz);
             if (out) {
                 float ezN[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) ezN[q] = dz[q] * ie[q];
+                for (int q = 0; q < 4; ++q) ezN[q] = __fmul_rn(dz[q], ie[q]);
                 float *ring = C.ring + s * C.slot_elems;
                 if (S.ring_full[0] >= 0) st4(ring + S.ring_full[0] + ro, ezN);
                 if (S.ring_full[1] >= 0) st4(ring + S.ring_full[1] + ro, hx);
@@ -561,7 +581,6 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_tm(
             if (bxE) st4(S.psi[2][pn] + ro, p2);
             if (byE) { lds4(yp3, t); st4(S.psi[3][pn] + ro, t); }
         }
-        __syncthreads();                                // records, exchange planes reused
     }
 }
 
@@ -582,7 +601,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
     const int par = C.par, pn = par ^ 1;
     const int cell = w * TB_C + 4 * lane;
     for (uint32_t k = 0; it < n_work; ++k, it += gridDim.x) {
-        if (!tb_begin<true>(k, L, C.err)) return;
+        const bool ok = tb_wait(*L.ctl, k & 1, C.err);
         const int4 wk = L.ctl->cur[k & 1];
         const TbMeta &M = L.meta[k & 1];
         const mtb_yee2d_struct &S = M.s;
@@ -592,8 +611,9 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
         tb_take(L.stage, 2, cell, dy);
         tb_take(L.stage, 3, cell, ix);
         tb_take(L.stage, 4, cell, iy);
-        tb_take_psi(L.stage + NF * TB_PLANE, wk.w, w, lane, p1, p2, L.yp);
-        __syncthreads();
+        const bool lean = wk.w & TBF_LEAN;
+        if (!lean) tb_take_psi(L.stage + NF * TB_PLANE, wk.w, w, lane, p1, p2, L.yp);
+        if (!__syncthreads_and(ok)) return;             // staging planes are free
         tb_next<true>(maps, C, work, n_work, it, k, L);
 
         const int nx = S.nx, ny = S.ny, P = S.pitch;
@@ -603,26 +623,6 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
         const bool rowIn = i >= 0 && i < nx;
         const bool hzRow = i >= 0 && i <= nx - 2, dyRow = i >= 1 && i <= nx - 2;
         const float dt = S.dt, rdx = 1.0f / S.dx;
-        unsigned mX = 0, mY = 0, mZ = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = jb + q;
-            if (hzRow && j >= 1 && j <= ny - 2) mX |= 1u << q;
-            if (dyRow && j >= 0 && j <= ny - 2) mY |= 1u << q;
-            if (hzRow && j >= 0 && j <= ny - 2) mZ |= 1u << q;
-        }
-        const bool bxH = hzRow && in_band(i, S.xband[0], S.xband[1]);
-        const bool bxE = dyRow && in_band(i, S.xband[2], S.xband[3]);
-        const float *xpr = L.xprof + (k & 1) * 4 * TB_R + w;
-        const float hxb = bxH ? xpr[0] : 1.f, hxa = bxH ? xpr[TB_R] : 0.f;
-        const float exb = bxE ? xpr[2 * TB_R] : 1.f, exa = bxE ? xpr[3 * TB_R] : 0.f;
-        const bool byE = act && hzRow && band4(jb, S.yband[2], S.yband[3]);
-        const bool byH = act && hzRow && band4(jb, S.yband[0], S.yband[1]);
-        // every lane of a tile that reaches a y layer runs the CPML arithmetic (inert
-        // profiles and zero memory off the layer give the plain update): no divergence
-        const bool yl = ((wk.w >> TBF_YSHIFT) & 3) != TBF_YNONE;
-        float *yp0 = L.yp + cell, *yp3 = L.yp + TB_PLANE + cell;
-        const float *pr = L.prof + (k & 1) * 4 * TB_C + 4 * lane;
         const bool outC = act && lane >= 1 && lane <= 30;
         const bool out = outC && rowIn && w >= TB_T && w < TB_T + TB_OUTR;
         const unsigned lmask = (unsigned)wk.w >> TBF_LINE_SHIFT;
@@ -631,8 +631,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                           i <= S.src_e.row_hi;
         const bool srcH = act && hzRow && S.src_h1.n > 0 && i >= S.src_h1.row_lo &&
                           i <= S.src_h1.row_hi;
-        if (wk.w & TBF_LEAN) {
-            // every cell of the tile is updated and no CPML term is active
+        if (lean) {
+            // every cell of the tile is updated and no CPML term is active (the one-barrier
+            // form of k_tb_tm needs the row below's Dy and 1/eps in registers too: it spilled,
+            // 94.7 against 85.9 us per launch of a 10-structure batch)
             float *rs0 = (out && S.ring_full[0] >= 0) ? C.ring + S.ring_full[0] + ro : nullptr;
             float *rs1 = (out && S.ring_full[1] >= 0) ? C.ring + S.ring_full[1] + ro : nullptr;
             float *rs2 = (out && S.ring_full[2] >= 0) ? C.ring + S.ring_full[2] + ro : nullptr;
@@ -647,13 +649,13 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float hm = (q == 0) ? hzL : hz[q - 1];
-                    dx[q] = dx[q] + dt * ((hz[q] - hm) * rdx);
-                    ex[q] = dx[q] * ix[q];
-                    dy[q] = dy[q] - dt * ((hz[q] - ha[q]) * rdx);
+                    dx[q] = __fmaf_rn(dt, tb_d(hz[q], hm, rdx), dx[q]);
+                    ex[q] = __fmul_rn(dx[q], ix[q]);
+                    dy[q] = __fmaf_rn(-dt, tb_d(hz[q], ha[q], rdx), dy[q]);
                 }
-                if (srcE) apply_cells(S.src_e, i, C.amp_e + s * C.ncols, jb, dy);
+                if (srcE) apply_cells_rn(S.src_e, i, C.amp_e + s * C.ncols, jb, dy);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) ey[q] = dy[q] * iy[q];
+                for (int q = 0; q < 4; ++q) ey[q] = __fmul_rn(dy[q], iy[q]);
                 st4(xy + cell, ey);
                 __syncthreads();
                 float eb[4];
@@ -662,12 +664,13 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                 const float exR = __shfl_down_sync(0xffffffffu, ex[0], 1);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float exn = (q < 3) ? ex[q + 1] : exR;
-                    const float dey = (eb[q] - ey[q]) * rdx;
-                    const float dex = (exn - ex[q]) * rdx;
-                    hz[q] = hz[q] - dt * (dey - dex);
+                    const float fy = __fmaf_rn(-dy[q], iy[q], eb[q]);
+                    const float fx = q == 3 ? __fmaf_rn(-dx[3], ix[3], exR)
+                                            : __fmaf_rn(dx[q < 3 ? q + 1 : 3], ix[q < 3 ? q + 1 : 3],
+                                                        -ex[q]);
+                    hz[q] = __fmaf_rn(-dt, __fmaf_rn(fy, rdx, -__fmul_rn(fx, rdx)), hz[q]);
                 }
-                if (srcH) apply_cells(S.src_h1, i, C.amp_h + s * C.ncols, jb, hz);
+                if (srcH) apply_cells_rn(S.src_h1, i, C.amp_h + s * C.ncols, jb, hz);
                 if (out) {
                     const int64_t so = s * C.slot_elems;
                     if (rs0) st4(rs0 + so, hz);
@@ -681,119 +684,112 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                     }
                 }
             }
-        } else
-        for (int s = 0; s < C.nsub; ++s) {
-            st4(xz + cell, hz);
-            __syncthreads();
-            float ha[4];
-            if (w > 0) lds4(xz + cell - TB_C, ha);
-            else zero4(ha);
-            const float hzL = __shfl_up_sync(0xffffffffu, hz[3], 1);       // lane 0: halo
-            // Dx / Ex(n+1/2)
-            if (yl) {
-                float p0[4], b[4], a[4];
-                lds4(yp0, p0);
-                lds4(pr + 2 * TB_C, b);
-                lds4(pr + 3 * TB_C, a);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float hm = (q == 0) ? hzL : hz[q - 1];
-                    const float d = (hz[q] - hm) * rdx;
-                    const float pv = b[q] * p0[q] + a[q] * d;
-                    const float dn = dx[q] + dt * (d + pv);
-                    const bool v = (mX >> q) & 1u;
-                    dx[q] = v ? dn : dx[q];
-                    p0[q] = v ? pv : p0[q];
-                }
-                st4(yp0, p0);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float hm = (q == 0) ? hzL : hz[q - 1];
-                    const float dn = dx[q] + dt * ((hz[q] - hm) * rdx);
-                    dx[q] = ((mX >> q) & 1u) ? dn : dx[q];
-                }
-            }
-            float ex[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) ex[q] = hzRow ? dx[q] * ix[q] : 0.f;
-            // Dy / Ey(n+1/2), source into Dy
-            if (bxE) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float d = (hz[q] - ha[q]) * rdx;
-                    const float pv = exb * p1[q] + exa * d;
-                    const float dn = dy[q] - dt * (d + pv);
-                    const bool v = (mY >> q) & 1u;
-                    dy[q] = v ? dn : dy[q];
-                    p1[q] = v ? pv : p1[q];
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float dn = dy[q] - dt * ((hz[q] - ha[q]) * rdx);
-                    dy[q] = ((mY >> q) & 1u) ? dn : dy[q];
-                }
-            }
-            if (srcE) apply_cells(S.src_e, i, C.amp_e + s * C.ncols, jb, dy);
-            float ey[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) ey[q] = rowIn ? dy[q] * iy[q] : 0.f;
-            st4(xy + cell, ey);
-            __syncthreads();
-            float eb[4];
-            if (w + 1 < TB_R) lds4(xy + cell + TB_C, eb);
-            else zero4(eb);
-            const float exR = __shfl_down_sync(0xffffffffu, ex[0], 1);     // lane 31: halo
-            // Hz(n+1)
-            if (yl || bxH) {
-                float p3[4], b3[4], a3[4];
-                if (yl) {
-                    lds4(yp3, p3);
-                    lds4(pr, b3);
-                    lds4(pr + TB_C, a3);
-                } else {
-                    zero4(p3); zero4(a3);
-                    b3[0] = b3[1] = b3[2] = b3[3] = 1.f;
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float exn = (q < 3) ? ex[q + 1] : exR;
-                    const float dey = (eb[q] - ey[q]) * rdx;
-                    const float dex = (exn - ex[q]) * rdx;
-                    const float q2 = hxb * p2[q] + hxa * dey;
-                    const float q3 = b3[q] * p3[q] + a3[q] * dex;
-                    const float cz = (dey + q2) - (dex + q3);
-                    const float hn = hz[q] - dt * cz;
-                    const bool v = (mZ >> q) & 1u;
-                    hz[q] = v ? hn : hz[q];
-                    p2[q] = v ? q2 : p2[q];
-                    p3[q] = v ? q3 : p3[q];
-                }
-                if (yl) st4(yp3, p3);
-            } else {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float exn = (q < 3) ? ex[q + 1] : exR;
-                    const float dey = (eb[q] - ey[q]) * rdx;
-                    const float dex = (exn - ex[q]) * rdx;
-                    const float hn = hz[q] - dt * (dey - dex);
-                    hz[q] = ((mZ >> q) & 1u) ? hn : hz[q];
-                }
-            }
-            if (srcH) apply_cells(S.src_h1, i, C.amp_h + s * C.ncols, jb, hz);
             if (out) {
-                float *ring = C.ring + s * C.slot_elems;
-                if (S.ring_full[0] >= 0) st4(ring + S.ring_full[0] + ro, hz);
-                if (S.ring_full[1] >= 0) st4(ring + S.ring_full[1] + ro, ex);
-                if (S.ring_full[2] >= 0) st4(ring + S.ring_full[2] + ro, ey);
-                if (lmask) {
-                    tb_sample(M.lines, lmask, MTB_C2_MAIN, i, jb, hz, ring);
-                    tb_sample(M.lines, lmask, MTB_C2_X, i, jb, ex, ring);
-                    tb_sample(M.lines, lmask, MTB_C2_Y, i, jb, ey, ring);
+                st4(S.f_main[pn] + ro, hz);
+                st4(S.f_x[pn] + ro, dx);
+                st4(S.f_y[pn] + ro, dy);
+            }
+            continue;
+        }
+        // validity as factors: columns in 1 / dx (Dx; Hz), rows in dt (Dy; Hz). Where a factor is
+        // zero the operands are too (walls, padding) or the row is not used. (In k_tb_tm this
+        // form spilled: 167 against 155 us per launch of 64 structures of 256 x 256.)
+        unsigned mX = 0, mZ = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = jb + q;
+            if (j >= 1 && j <= ny - 2) mX |= 1u << q;
+            if (j >= 0 && j <= ny - 2) mZ |= 1u << q;
+        }
+        const float ty = dyRow ? dt : 0.f, tz = hzRow ? dt : 0.f;
+        const bool bxH = hzRow && in_band(i, S.xband[0], S.xband[1]);
+        const bool bxE = dyRow && in_band(i, S.xband[2], S.xband[3]);
+        const float *xpr = L.xprof + (k & 1) * 4 * TB_R + w;
+        const float hxb = bxH ? xpr[0] : 1.f, hxa = bxH ? xpr[TB_R] : 0.f;
+        const float exb = bxE ? xpr[2 * TB_R] : 1.f, exa = bxE ? xpr[3 * TB_R] : 0.f;
+        const bool byE = act && hzRow && band4(jb, S.yband[2], S.yband[3]);
+        const bool byH = act && hzRow && band4(jb, S.yband[0], S.yband[1]);
+        // every lane of a tile that reaches a y layer runs the CPML arithmetic (inert
+        // profiles and zero memory off the layer give the plain update): no divergence
+        const bool yl = ((wk.w >> TBF_YSHIFT) & 3) != TBF_YNONE;
+        float *yp0 = L.yp + cell, *yp3 = L.yp + TB_PLANE + cell;
+        const float *pr = L.prof + (k & 1) * 4 * TB_C + 4 * lane;
+        auto steps = [&](auto ylayer) {
+            constexpr bool YL = decltype(ylayer)::value;
+            for (int s = 0; s < C.nsub; ++s) {
+                st4(xz + cell, hz);
+                __syncthreads();
+                float ha[4];
+                if (w > 0) lds4(xz + cell - TB_C, ha);
+                else zero4(ha);
+                const float hzL = __shfl_up_sync(0xffffffffu, hz[3], 1);       // lane 0: halo
+                // Dx / Ex(n+1/2)
+                float p[4], b[4], a[4], ex[4], ey[4];
+                if (YL) { lds4(yp0, p); lds4(pr + 2 * TB_C, b); lds4(pr + 3 * TB_C, a); }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float d = tb_d(hz[q], q > 0 ? hz[q > 0 ? q - 1 : 0] : hzL,
+                                         ((mX >> q) & 1u) ? rdx : 0.f);
+                    dx[q] = __fmaf_rn(dt, YL ? tb_cpml(d, b[q], a[q], p[q]) : d, dx[q]);
+                    ex[q] = __fmul_rn(dx[q], ix[q]);
+                }
+                if (YL) st4(yp0, p);
+                // Dy / Ey(n+1/2), source into Dy
+                if (bxE) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        dy[q] = __fmaf_rn(-ty, tb_cpml(tb_d(hz[q], ha[q], rdx), exb, exa, p1[q]), dy[q]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        dy[q] = __fmaf_rn(-ty, tb_d(hz[q], ha[q], rdx), dy[q]);
+                }
+                if (srcE) apply_cells_rn(S.src_e, i, C.amp_e + s * C.ncols, jb, dy);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ey[q] = __fmul_rn(dy[q], iy[q]);
+                st4(xy + cell, ey);
+                __syncthreads();
+                float eb[4];
+                if (w + 1 < TB_R) lds4(xy + cell + TB_C, eb);
+                else zero4(eb);
+                const float exR = __shfl_down_sync(0xffffffffu, ex[0], 1);     // lane 31: halo
+                // Hz(n+1)
+                if (YL) { lds4(yp3, p); lds4(pr, b); lds4(pr + TB_C, a); }
+                if (YL || bxH) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float cz = ((mZ >> q) & 1u) ? rdx : 0.f;
+                        const float dey = tb_d(eb[q], ey[q], cz);
+                        const float dex = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], cz);
+                        const float t = bxH ? tb_cpml(dey, hxb, hxa, p2[q]) : dey;
+                        const float u = YL ? tb_cpml(dex, b[q], a[q], p[q]) : dex;
+                        hz[q] = __fmaf_rn(-tz, __fsub_rn(t, u), hz[q]);
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float cz = ((mZ >> q) & 1u) ? rdx : 0.f;
+                        const float dex = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], cz);
+                        hz[q] = __fmaf_rn(-tz, __fmaf_rn(__fsub_rn(eb[q], ey[q]), cz, -dex), hz[q]);
+                    }
+                }
+                if (YL) st4(yp3, p);
+                if (srcH) apply_cells_rn(S.src_h1, i, C.amp_h + s * C.ncols, jb, hz);
+                if (out) {
+                    float *ring = C.ring + s * C.slot_elems;
+                    if (S.ring_full[0] >= 0) st4(ring + S.ring_full[0] + ro, hz);
+                    if (S.ring_full[1] >= 0) st4(ring + S.ring_full[1] + ro, ex);
+                    if (S.ring_full[2] >= 0) st4(ring + S.ring_full[2] + ro, ey);
+                    if (lmask) {
+                        tb_sample(M.lines, lmask, MTB_C2_MAIN, i, jb, hz, ring);
+                        tb_sample(M.lines, lmask, MTB_C2_X, i, jb, ex, ring);
+                        tb_sample(M.lines, lmask, MTB_C2_Y, i, jb, ey, ring);
+                    }
                 }
             }
-        }
+        };
+        if (yl) steps(std::true_type{});
+        else steps(std::false_type{});
         if (out) {
             st4(S.f_main[pn] + ro, hz);
             st4(S.f_x[pn] + ro, dx);
@@ -804,7 +800,6 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
             if (bxH) st4(S.psi[2][pn] + ro, p2);
             if (byH) { lds4(yp3, t); st4(S.psi[3][pn] + ro, t); }
         }
-        __syncthreads();
     }
 }
 
