@@ -603,6 +603,10 @@ int mtb_yee3d_adjoint_psi_layers(mtb_yee3d_adjoint *p, int32_t only_layers);
 int64_t mtb_yee3d_adjoint_last_launches(const mtb_yee3d_adjoint *p);
 void mtb_yee3d_adjoint_destroy(mtb_yee3d_adjoint *p);
 
+/* Plans take their scratch from a pool that keeps at most 256 MB of device and 16 MB of
+ * pinned host memory after they are destroyed; this frees what it keeps. */
+void mtb_release_scratch(void);
+
 /* ------------------------------------------------------------ layout */
 
 /* Strided copy of an n0 x n1 x n2 block between a dense reference array

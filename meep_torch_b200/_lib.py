@@ -163,6 +163,7 @@ SIGNATURES = {
     "mtb_pack": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, vp,
                            C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                            C.c_int64, C.c_int64, vp]),
+    "mtb_release_scratch": (None, []),
     "mtb_pack_eps": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, vp, vp, vp]),
     "mtb_zero": (C.c_int, [C.POINTER(C.c_uint64), C.POINTER(C.c_int64), C.c_int32, vp]),
     "mtb_unpack": (C.c_int, [vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,

@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <mutex>
 #include <vector>
 
 #include "mtb_common.cuh"
@@ -70,6 +71,120 @@ void LaunchTimer::release() {
     for (auto e : pool) cudaEventDestroy(e);
     pool.clear();
     used = 0;
+}
+
+// ------------------------------------------------------------ plan scratch
+
+namespace {
+struct Kept {
+    void *p;
+    size_t bytes;
+    int dev;
+};
+struct ScratchPool {
+    std::mutex mu;
+    std::vector<Kept> kept;          // oldest first
+    size_t held = 0;
+};
+// never destroyed: plans may be closed while the process exits
+ScratchPool &scratch_pool(bool host) {
+    static ScratchPool *pools = new ScratchPool[2];
+    return pools[host];
+}
+cudaError_t raw_alloc(bool host, void **p, size_t n) {
+    return host ? cudaMallocHost(p, n) : cudaMalloc(p, n);
+}
+void raw_free(bool host, void *p) {
+    if (host) cudaFreeHost(p);
+    else cudaFree(p);
+}
+// makes `dev` current for its lifetime
+struct OnDevice {
+    int before = 0;
+    bool moved = false;
+    explicit OnDevice(int dev) {
+        moved = cudaGetDevice(&before) == cudaSuccess && before != dev &&
+                cudaSetDevice(dev) == cudaSuccess;
+    }
+    ~OnDevice() {
+        if (moved) cudaSetDevice(before);
+    }
+};
+// frees the oldest kept blocks until at most `keep` bytes stay
+void scratch_trim(bool host, size_t keep) {
+    ScratchPool &P = scratch_pool(host);
+    for (;;) {
+        Kept k{};
+        {
+            std::lock_guard<std::mutex> lock(P.mu);
+            if (P.held <= keep || P.kept.empty()) return;
+            k = P.kept.front();
+            P.kept.erase(P.kept.begin());
+            P.held -= k.bytes;
+        }
+        OnDevice on(k.dev);
+        raw_free(host, k.p);
+    }
+}
+}  // namespace
+
+int scratch_get(bool host, size_t n, void **p, size_t *bytes, int *dev) {
+    *p = nullptr;
+    *bytes = 0;
+    MTB_CUDA_TRY(cudaGetDevice(dev));
+    if (n == 0) return MTB_OK;
+    const size_t unit = n < ((size_t)1 << 20) ? 512 : (size_t)1 << 16;
+    n = (n + unit - 1) / unit * unit;
+    {
+        ScratchPool &P = scratch_pool(host);
+        std::lock_guard<std::mutex> lock(P.mu);
+        int best = -1;
+        for (int k = 0; k < (int)P.kept.size(); ++k) {
+            const Kept &b = P.kept[k];
+            if (b.dev == *dev && b.bytes >= n && b.bytes <= 2 * n &&
+                (best < 0 || b.bytes < P.kept[best].bytes))
+                best = k;
+        }
+        if (best >= 0) {
+            *p = P.kept[best].p;
+            *bytes = P.kept[best].bytes;
+            P.held -= *bytes;
+            P.kept.erase(P.kept.begin() + best);
+            return MTB_OK;
+        }
+    }
+    cudaError_t e = raw_alloc(host, p, n);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_trim(host, 0);
+        e = raw_alloc(host, p, n);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        return fail(MTB_CUDA_ERROR, "%s(%zu) failed: %s", host ? "cudaMallocHost" : "cudaMalloc", n,
+                    cudaGetErrorString(e));
+    }
+    *bytes = n;
+    return MTB_OK;
+}
+
+void scratch_put(bool host, void *p, size_t bytes, int dev) {
+    OnDevice on(dev);
+    // work that uses the block may still run, on any stream
+    bool keep = bytes <= SCRATCH_KEEP[host] && cudaDeviceSynchronize() == cudaSuccess;
+    if (keep) {
+        ScratchPool &P = scratch_pool(host);
+        std::lock_guard<std::mutex> lock(P.mu);
+        try {
+            P.kept.push_back({p, bytes, dev});
+            P.held += bytes;
+        } catch (...) {
+            keep = false;
+        }
+    }
+    if (keep) scratch_trim(host, SCRATCH_KEEP[host]);
+    else raw_free(host, p);
 }
 
 // ------------------------------------------------------------ layout kernels
@@ -656,6 +771,11 @@ int64_t mtb_struct_size(int32_t which) {
         case 8: return sizeof(mtb_adj3d_buffers);
         default: return -1;
     }
+}
+
+void mtb_release_scratch(void) {
+    scratch_trim(false, 0);
+    scratch_trim(true, 0);
 }
 
 int mtb_pack(const float *src, int64_t n0, int64_t n1, int64_t n2, int64_t s0, int64_t s1,
