@@ -614,6 +614,7 @@ __global__ void __launch_bounds__(32 * AROWS) k_adj_te_hzh(const __grid_constant
 using namespace mtb;
 
 struct mtb_yee2d_adjoint {
+    StreamMarks marks;             // streams its work runs on
     mtb_yee2d_struct s{};
     mtb_adj2d_buffers b{};
     DftState dft;
@@ -784,6 +785,7 @@ int mtb_yee2d_adjoint_run(mtb_yee2d_adjoint *p, int64_t t0, int32_t k, const flo
     if (!p) return fail(MTB_INVALID_ARG, "adjoint plan is null");
     p->last_launches = 0;
     if (k <= 0) return MTB_OK;
+    const MarkUse use(p->marks, stream);
     if (k > p->dft.slots) return fail(MTB_INVALID_ARG, "k %d > ring slots %d", k, p->dft.slots);
     if (!rec_offset_in) return fail(MTB_INVALID_ARG, "adjoint: null record offsets");
     const int64_t rec_offset[2] = {rec_offset_in[0],
@@ -840,6 +842,7 @@ void mtb_yee2d_adjoint_destroy(mtb_yee2d_adjoint *p) {
     if (!p) return;
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     if (p->cap) cudaStreamDestroy(p->cap);
+    const ScratchIdle scratch(p->marks.wait());
     p->dft.release();
     delete p;
 }

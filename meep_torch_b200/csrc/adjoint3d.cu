@@ -434,6 +434,7 @@ __global__ void __launch_bounds__(A3_T) k_adj3_eps(const __grid_constant__ Adj3 
 using namespace mtb;
 
 struct mtb_yee3d_adjoint {
+    StreamMarks marks;             // streams its work runs on
     mtb_yee3d_struct s{};
     Adj3 a{};
     DftState dft;
@@ -548,6 +549,7 @@ int mtb_yee3d_adjoint_run(mtb_yee3d_adjoint *p, int64_t t0, int32_t k, const flo
     if (!p) return fail(MTB_INVALID_ARG, "3D adjoint plan is null");
     p->last_launches = 0;
     if (k <= 0) return MTB_OK;
+    const MarkUse use(p->marks, stream);
     if (k > p->dft.slots) return fail(MTB_INVALID_ARG, "k %d > ring slots %d", k, p->dft.slots);
     if (!rec || (reinterpret_cast<uintptr_t>(rec) & 15) || (rec_comp_stride & 3) ||
         (rec_slot_stride & 3))
@@ -613,6 +615,7 @@ int64_t mtb_yee3d_adjoint_last_launches(const mtb_yee3d_adjoint *p) {
 
 void mtb_yee3d_adjoint_destroy(mtb_yee3d_adjoint *p) {
     if (!p) return;
+    const ScratchIdle scratch(p->marks.wait());
     p->dft.release();
     p->s_d.release();
     p->pstart_d.release();

@@ -169,10 +169,13 @@ int scratch_get(bool host, size_t n, void **p, size_t *bytes, int *dev) {
     return MTB_OK;
 }
 
+static thread_local bool scratch_idle = false;
+ScratchIdle::ScratchIdle(bool idle) { scratch_idle = idle; }
+ScratchIdle::~ScratchIdle() { scratch_idle = false; }
+
 void scratch_put(bool host, void *p, size_t bytes, int dev) {
     OnDevice on(dev);
-    // work that uses the block may still run, on any stream
-    bool keep = bytes <= SCRATCH_KEEP[host] && cudaDeviceSynchronize() == cudaSuccess;
+    bool keep = scratch_idle && bytes <= SCRATCH_KEEP[host];
     if (keep) {
         ScratchPool &P = scratch_pool(host);
         std::lock_guard<std::mutex> lock(P.mu);

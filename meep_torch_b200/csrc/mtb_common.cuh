@@ -40,8 +40,10 @@ void count_launch(int64_t n = 1);
 // Plan scratch comes from a bounded pool, so that building and closing a plan does not pay
 // cudaMalloc / cudaFree (and their pinned forms) a dozen times: these took 1.3 of the 3.3 ms of
 // a 200-step run of a small plan, and up to 10 ms where other programs use the driver too.
-// A block goes back after the device has finished (as cudaFree waits), so any thread, stream or
-// plan of that device may take it next; contents are not kept or cleared. At most
+// A block goes back only when the work of every stream its plan ran on has finished
+// (StreamMarks, ScratchIdle; not by a device-wide wait, which breaks graph captures of other
+// threads), so any thread, stream or plan of that device may take it next; contents are not
+// kept or cleared. Without that knowledge it is freed, as cudaFree waits by itself. At most
 // SCRATCH_KEEP bytes stay (the oldest blocks are freed first), none are kept when an
 // allocation fails, and mtb_release_scratch() frees all.
 constexpr size_t SCRATCH_KEEP[2] = {(size_t)256 << 20, (size_t)16 << 20};   // device, pinned
@@ -69,6 +71,58 @@ struct ScratchBuf {
 };
 using DevBuf = ScratchBuf<false>;
 using HostBuf = ScratchBuf<true>;
+
+// The streams a plan has queued work on, each with an event behind its latest use.
+struct StreamMarks {
+    struct One {
+        cudaStream_t st;
+        cudaEvent_t ev;
+    };
+    std::vector<One> uses;
+    bool unknown = false;            // captured by a caller, or an event failed: cannot tell
+    void mark(cudaStream_t st) noexcept {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (unknown) return;
+        unknown = true;
+        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+            return;
+        cudaEvent_t ev = nullptr;
+        for (const One &u : uses)
+            if (u.st == st) ev = u.ev;
+        if (!ev) {
+            if (uses.size() >= 16) return;
+            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return;
+            try {
+                uses.push_back({st, ev});
+            } catch (...) {
+                cudaEventDestroy(ev);
+                return;
+            }
+        }
+        unknown = cudaEventRecord(ev, st) != cudaSuccess;
+    }
+    // waits for all of it; false if that cannot be told
+    bool wait() noexcept {
+        for (const One &u : uses) {
+            if (!unknown && cudaEventSynchronize(u.ev) != cudaSuccess) unknown = true;
+            cudaEventDestroy(u.ev);
+        }
+        uses.clear();
+        return !unknown;
+    }
+};
+// marks the plan's use of a stream when an entry point returns, by any path
+struct MarkUse {
+    StreamMarks &m;
+    cudaStream_t st;
+    MarkUse(StreamMarks &marks, void *stream) : m(marks), st((cudaStream_t)stream) {}
+    ~MarkUse() { m.mark(st); }
+};
+// while it lives, buffers that this thread releases are known to be idle (if `idle`)
+struct ScratchIdle {
+    explicit ScratchIdle(bool idle);
+    ~ScratchIdle();
+};
 
 // Programmatic dependent launch, for chains of short step kernels: a kernel launched by
 // launch_pdl may start while its predecessor still runs, once every block of that one has

@@ -2089,6 +2089,8 @@ using namespace mtb;
 struct mtb_yee2d_plan {
     int n_structs = 0;
     DevBuf structs_d, work_d, amp_d, err_d;
+    mutable StreamMarks marks;         // streams its work runs on
+    mutable bool ring_out = false;     // the ring was handed out (mtb_yee2d_ring)
     PinnedPair amp_h;
     int n_work = 0;
     int n_work_tm = 0;                 // work items [0, n_work_tm) are TM, the rest TE
@@ -3337,6 +3339,7 @@ int mtb_yee2d_run(mtb_yee2d_plan *p, int64_t t0, int32_t k, const double *coef_e
     if (k < 0) return fail(MTB_INVALID_ARG, "k < 0");
     p->last_launches = 0;
     if (k == 0) return MTB_OK;
+    const MarkUse use(p->marks, stream);
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
     // the row march's bounded waits may have raised the error flag (the TB and resident
@@ -3510,6 +3513,7 @@ int mtb_yee2d_ring_gather(const mtb_yee2d_plan *p, const int64_t *offsets, int32
     if (!offsets || !out || !p->dft.ring_d.p)
         return fail(MTB_INVALID_ARG, "ring gather: null offsets, output or ring");
     const int64_t n = (int64_t)n_off * n_slots;
+    const MarkUse use(p->marks, stream);
     k_ring_gather<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
         p->dft.ring_d.as<float>(), p->dft.slot_elems, offsets, n_off, n_slots, out);
     MTB_CHECK_LAUNCH();
@@ -3518,7 +3522,10 @@ int mtb_yee2d_ring_gather(const mtb_yee2d_plan *p, const int64_t *offsets, int32
 
 int mtb_yee2d_ring(const mtb_yee2d_plan *p, float **ring, int64_t *slot_elems, int32_t *slots) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
-    if (ring) *ring = const_cast<float *>(p->dft.ring_d.as<float>());
+    if (ring) {
+        *ring = const_cast<float *>(p->dft.ring_d.as<float>());
+        p->ring_out = true;
+    }
     if (slot_elems) *slot_elems = p->dft.slot_elems;
     if (slots) *slots = p->dft.slots;
     return MTB_OK;
@@ -3529,6 +3536,9 @@ void mtb_yee2d_plan_destroy(mtb_yee2d_plan *p) {
     for (int q = 0; q < 2; ++q)
         if (p->gexec[q]) cudaGraphExecDestroy(p->gexec[q]);
     if (p->cap) cudaStreamDestroy(p->cap);
+    const bool idle = p->marks.wait();
+    if (p->ring_out) p->dft.ring_d.release();        // others may still read it
+    const ScratchIdle scratch(idle);
     p->stage_d.release();
     p->rb_work_d.release();
     p->rb_meta_d.release();

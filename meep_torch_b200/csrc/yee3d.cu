@@ -843,6 +843,7 @@ using namespace mtb;
 struct mtb_yee3d_plan {
     mtb_yee3d_struct s{};
     DevBuf s_d, pstart_d, amp_d;
+    StreamMarks marks;             // streams its work runs on
     PinnedPair amp_h;
     int rows = 32;
     int nzw = 1;
@@ -1458,6 +1459,7 @@ extern "C" {
 
 int mtb_yee3d_run(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
+    const MarkUse use(p->marks, stream);
     if (k < 0) return fail(MTB_INVALID_ARG, "k < 0");
     p->last_launches = 0;
     if (k == 0) return MTB_OK;
@@ -1530,6 +1532,7 @@ int mtb_yee3d_set_slab(mtb_yee3d_plan *p, int32_t own_lo, int32_t own_hi) {
 
 int mtb_yee3d_begin(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
+    const MarkUse use(p->marks, stream);
     if (int rc = need_split(p, "half steps")) return rc;
     if (k <= 0) return fail(MTB_INVALID_ARG, "k must be > 0");
     p->last_launches = 0;
@@ -1538,6 +1541,7 @@ int mtb_yee3d_begin(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef
 
 int mtb_yee3d_half(mtb_yee3d_plan *p, int32_t part, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
+    const MarkUse use(p->marks, stream);
     if (p->c_s >= p->c_k) return fail(MTB_INVALID_ARG, "no staged step left (mtb_yee3d_begin)");
     if (part != p->c_half)
         return fail(MTB_INVALID_ARG, "half %d out of order (expected %d)", part, p->c_half);
@@ -1557,6 +1561,7 @@ int mtb_yee3d_half(mtb_yee3d_plan *p, int32_t part, void *stream) {
 int mtb_yee3d_run_record(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, float *rec,
                          int64_t rec_comp_stride, int64_t rec_slot_stride, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
+    const MarkUse use(p->marks, stream);
     if (int rc = need_split(p, "recorded steps")) return rc;
     if (k < 0) return fail(MTB_INVALID_ARG, "k < 0");
     if (!rec || (reinterpret_cast<uintptr_t>(rec) & 15) || (rec_comp_stride & 3) ||
@@ -1615,6 +1620,7 @@ int64_t mtb_yee3d_last_launches(const mtb_yee3d_plan *p) { return p ? p->last_la
 
 void mtb_yee3d_plan_destroy(mtb_yee3d_plan *p) {
     if (!p) return;
+    const ScratchIdle scratch(p->marks.wait());
     p->s_d.release();
     p->pstart_d.release();
     p->amp_d.release();

@@ -51,18 +51,21 @@ def test_threads_share_the_pool():
     want, bad = _run("tm", 120, 100, 64), []
 
     def work():
-        with torch.cuda.stream(torch.cuda.Stream()):
-            for _ in range(4):
-                if not _same(_run("tm", 120, 100, 64), want):
-                    bad.append(1)
-            torch.cuda.current_stream().synchronize()
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(12):
+                    if not _same(_run("tm", 120, 100, 64), want):
+                        bad.append("differs")
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:      # a thread's exception would go unseen
+            bad.append(repr(e))
 
     ts = [threading.Thread(target=work) for _ in range(3)]
     for t in ts:
         t.start()
     for t in ts:
         t.join()
-    assert not bad
+    assert not bad, bad
 
 
 def test_kept_memory_is_bounded_and_given_back():
