@@ -460,6 +460,10 @@ int mtb_yee2d_adjoint_create(const mtb_yee2d_struct *s, const mtb_adj2d_buffers 
  * rec_offset[1]. */
 int mtb_yee2d_adjoint_run(mtb_yee2d_adjoint *p, int64_t t0, int32_t k, const float *rec,
                           int64_t rec_slot_elems, const int64_t *rec_offset, void *stream);
+/* only_layers != 0 (before the first run): g_psi is kept inside the CPML layers only
+ * (elsewhere it feeds nothing back), which saves its traffic outside them. Default 0:
+ * g_psi is d J / d psi everywhere. */
+int mtb_yee2d_adjoint_psi_layers(mtb_yee2d_adjoint *p, int32_t only_layers);
 int64_t mtb_yee2d_adjoint_last_launches(const mtb_yee2d_adjoint *p);
 void mtb_yee2d_adjoint_destroy(mtb_yee2d_adjoint *p);
 

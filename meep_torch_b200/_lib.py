@@ -154,6 +154,7 @@ SIGNATURES = {
                                            C.POINTER(PhaseGroup), C.c_int32, C.c_int64,
                                            C.c_int32, C.POINTER(vp)]),
     "mtb_yee3d_adjoint_run": (C.c_int, [vp, C.c_int64, C.c_int32, vp, C.c_int64, C.c_int64, vp]),
+    "mtb_yee2d_adjoint_psi_layers": (C.c_int, [vp, C.c_int32]),
     "mtb_yee3d_adjoint_psi_layers": (C.c_int, [vp, C.c_int32]),
     "mtb_yee3d_adjoint_last_launches": (C.c_int64, [vp]),
     "mtb_yee3d_adjoint_destroy": (None, [vp]),

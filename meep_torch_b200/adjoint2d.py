@@ -151,6 +151,8 @@ class GradRun2D:
                                              regs if nreg else None, nreg, eng.groups,
                                              eng.n_groups, eng.ring_elems, self.sub,
                                              C.byref(adj)), "mtb_yee2d_adjoint_create")
+        # d J / d psi is not returned: it is only needed where it feeds back
+        L.check(lib.mtb_yee2d_adjoint_psi_layers(adj, 1), "mtb_yee2d_adjoint_psi_layers")
         keep = [gaccs, g, gpsi, tmp, geps, gpol, gpol_y, gcut, gb, gmp]
         stream = eng._sptr()
         try:

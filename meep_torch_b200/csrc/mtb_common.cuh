@@ -20,6 +20,11 @@ void set_error(const char *fmt, ...);
 int fail(int code, const char *fmt, ...);
 void count_launch(int64_t n = 1);
 
+// CPML band of a 2D profile (device arrays of n nodes): nodes with a != 0 or b != 1 satisfy
+// k < lo_end or k >= hi_start (s: structure number for messages)
+int profile_band(const float *b_d, const float *a_d, int n, int32_t &lo_end, int32_t &hi_start,
+                 int s);
+
 #define MTB_CUDA_TRY(expr)                                                    \
     do {                                                                      \
         cudaError_t e_ = (expr);                                              \

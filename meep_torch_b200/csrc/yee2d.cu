@@ -2431,8 +2431,8 @@ static int cell_rows(mtb_cells &cl, int rows, int s) {
 // every active node (a != 0 or b != 1) of the low half, [hi_begin, n) every
 // active node of the high half. Inert nodes inside a band are harmless (their
 // CPML memory stays zero and the effective derivative is the plain one).
-static int profile_band(const float *b_d, const float *a_d, int n, int32_t &lo_end,
-                        int32_t &hi_begin, int s) {
+int mtb::profile_band(const float *b_d, const float *a_d, int n, int32_t &lo_end,
+                      int32_t &hi_begin, int s) {
     std::vector<float> b(n), a(n);
     cudaError_t e = cudaMemcpy(b.data(), b_d, sizeof(float) * n, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(a.data(), a_d, sizeof(float) * n, cudaMemcpyDeviceToHost);
