@@ -166,14 +166,15 @@ class GradRun2D:
                 if rec is not None:
                     rec.close()
                 rec = Engine2D([(self.state0, self.coeffs, self.source, rec_mons)],
-                               phase_mode=self.phase_mode, ring_slots=self.sub, graph=False)
+                               phase_mode=self.phase_mode, ring_slots=self.sub, graph=False,
+                               fold=False)
 
             def restored(snap):
                 nonlocal rec
                 if rec is None:
                     rec = Engine2D([(zero, self.coeffs, self.source, rec_mons)],
                                    phase_mode=self.phase_mode, ring_slots=self.sub,
-                                   graph=False)
+                                   graph=False, fold=False)
                 rec.restore(0, snap)
 
             for c in range(len(self.chunks) - 1, -1, -1):

@@ -187,8 +187,10 @@ class Engine2D:
 
     def __init__(self, items, *, phase_mode: str = "exact", rows_per_warp: int = 0,
                  ring_slots: int = 0, variant: int = 0, graph: bool = True, stream=None,
-                 arena: bool = False):
+                 arena: bool = False, fold: bool = True):
         self.lib = L.load()
+        self.fold = bool(fold)           # False: samples stay in the ring (mtb_yee2d_ring),
+        #                                  no accumulator is formed
         self.use_arena = bool(arena)
         self.items = [_Item(*it) for it in items]
         _need(len(self.items) > 0, "empty batch")
@@ -688,7 +690,9 @@ class Engine2D:
             self._make_arena(structs)
         tun = L.Tuning(rows_per_warp, ring_slots, 0 if graph else -1, variant)
         plan = C.c_void_p()
-        L.check(lib.mtb_yee2d_plan_create(structs, len(self.items), reg_arr, len(regions),
+        L.check(lib.mtb_yee2d_plan_create(structs, len(self.items),
+                                          reg_arr if self.fold else None,
+                                          len(regions) if self.fold else 0,
                                           grp_arr, len(groups), ring, amp_cols, C.byref(tun),
                                           C.byref(plan)), "mtb_yee2d_plan_create")
         self.plan = plan
