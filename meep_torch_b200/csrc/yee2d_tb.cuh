@@ -208,18 +208,22 @@ __device__ __forceinline__ void tb_issue(const CUtensorMap *__restrict__ maps, c
 }
 
 // Bounded wait of each thread for tile k's copies (which also acquires them). False if it
-// expired; the caller's next barrier makes that block-uniform.
+// expired; the caller's next barrier makes that block-uniform, so any thread that ran out
+// raises the error flag: the others, thread 0 among them, may have seen the copies land. The
+// clock runs on while the context is switched out, so an expired wait looks once more.
 __device__ __forceinline__ bool tb_wait(TbCtl &ctl, uint32_t parity, int *err) {
     bool ok = mbar_try_wait(&ctl.bar, parity);
     if (!ok) {
         const unsigned long long t0 = gtimer();
         while (!(ok = mbar_try_wait(&ctl.bar, parity)) && gtimer() - t0 < WAIT_NS) {
         }
-        if (!ok && threadIdx.x == 0) {
+        if (!ok) ok = mbar_try_wait(&ctl.bar, parity);
+        if (!ok) {
             atomicExch(err, 1);
             // let the copies in flight land before the block exits (bounded)
             const unsigned long long t1 = gtimer();
-            while (!mbar_try_wait(&ctl.bar, parity) && gtimer() - t1 < WAIT_NS) {
+            while (threadIdx.x == 0 && !mbar_try_wait(&ctl.bar, parity) &&
+                   gtimer() - t1 < WAIT_NS) {
             }
         }
     }
