@@ -164,6 +164,7 @@ class GradRun2D:
             def from_state0():      # the initial state as imported (explicit Ez honoured)
                 nonlocal rec
                 if rec is not None:
+                    rec.check()
                     rec.close()
                 rec = Engine2D([(self.state0, self.coeffs, self.source, rec_mons)],
                                phase_mode=self.phase_mode, ring_slots=self.sub, graph=False,
@@ -205,6 +206,7 @@ class GradRun2D:
                     L.check(lib.mtb_yee2d_adjoint_run(adj, u0, uk, ring, selems.value, offs2,
                                                       stream), "mtb_yee2d_adjoint_run")
             if rec is not None:
+                rec.check()
                 rec.close()
         finally:
             lib.mtb_yee2d_adjoint_destroy(adj)

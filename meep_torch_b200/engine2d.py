@@ -916,8 +916,9 @@ class Engine2D:
         return out
 
     def check(self):
-        """Raise if a bounded wait of a staging kernel (row march, temporally blocked
-        tiles) expired; synchronises the plan's stream (once per run)."""
+        """Raise if a bounded wait of a kernel (row march, temporally blocked or resident
+        tiles) expired, so that fields and samples are incomplete; synchronises the plan's
+        stream (once per run)."""
         if not getattr(self, "_checked", False):
             L.check(self.lib.mtb_yee2d_check(self.plan, self._sptr()), "mtb_yee2d_check")
             self._checked = True
@@ -1008,6 +1009,12 @@ class Engine2D:
             psi_Hxy=self._unpack(ps[3][cur], (nx_e, ny_e), (xoff, yoff)))
 
     def accumulators(self, b: int = 0):
+        """Structure b's accumulators, one per monitor (the plan's own buffers). Checks the
+        run first (see check()), unless the plan's stream is being captured."""
+        with torch.cuda.stream(self.stream):
+            capturing = torch.cuda.is_current_stream_capturing()
+        if not capturing:
+            self.check()
         return list(self.items[b].accs)
 
     def close(self):

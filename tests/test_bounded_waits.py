@@ -67,3 +67,100 @@ def test_landed_copies_are_taken(wait, thread):
     assert wait(thread, 40, 0) == (1, 0)         # while waiting
     # between a poll and a reading of the clock that lies past the limit
     assert wait(thread, 2, 5000) == (1, 0)
+
+
+# ------------------------------------------------------------------ who reads the flag
+class _Lib:
+    """Every entry point succeeds, but the plans named in ``timed_out`` report a timeout."""
+
+    def __init__(self, timed_out=()):
+        self.timed_out = set(timed_out)
+
+    def mtb_yee2d_check(self, plan, stream):
+        return 3 if plan in self.timed_out else 0
+
+    def mtb_last_error(self):
+        return b"a bounded wait expired"
+
+    def __getattr__(self, name):
+        return lambda *a: 0
+
+
+@pytest.fixture
+def fake(monkeypatch):
+    import torch
+
+    from meep_torch_b200 import _lib as L
+    lib = _Lib()
+    monkeypatch.setattr(L, "load", lambda: lib)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    return lib
+
+
+def _engine(lib, plan, nx=6, ny=8):
+    import types
+
+    import torch
+
+    from meep_torch_b200 import _lib as L
+    from meep_torch_b200.engine2d import Engine2D
+    e = Engine2D.__new__(Engine2D)
+    e.lib, e.plan, e.stream, e.device = lib, plan, None, torch.device("cpu")
+    e._sptr = lambda: 0
+    e.items = [types.SimpleNamespace(nx=nx, ny=ny, accs=[torch.zeros(3)])]
+    e.structs = (L.Yee2DStruct * 1)()
+    e.structs[0].pitch = ny
+    e.regions, e.n_regions = None, 0
+    e.groups, e.n_groups, e.ring_elems = None, 0, 0
+    e._pack = lambda *a: torch.zeros(nx, ny)
+    e._unpack = lambda *a: torch.zeros(nx, ny)
+    e.run = lambda t0, k: setattr(e, "_checked", False)
+    e.snapshot = lambda b: []
+    e.restore = lambda b, snap: None
+    e._checked = False
+    return e
+
+
+def test_accumulators_report_a_timeout(fake, monkeypatch):
+    import torch
+
+    from meep_torch_b200._lib import MtbError
+    fake.timed_out = {"p"}
+    e = _engine(fake, "p")
+    with pytest.raises(MtbError, match="bounded wait"):
+        e.accumulators(0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert len(e.accumulators(0)) == 1               # no synchronisation in a capture
+    e.plan = None
+
+
+@pytest.mark.parametrize("late", [None, "rec0", "rec1", "rec2"])
+def test_gradient_reports_a_timeout_of_any_recording_plan(fake, monkeypatch, late):
+    """The chunks are recorded anew by up to three plans, two of them closed on the way."""
+    import collections
+    import types
+
+    import torch
+
+    from meep_torch_b200 import adjoint2d
+    from meep_torch_b200._lib import MtbError
+    plans = []
+
+    def recording(items, **kw):
+        plans.append(f"rec{len(plans)}")
+        return _engine(fake, plans[-1])
+    monkeypatch.setattr(adjoint2d, "Engine2D", recording)
+    monkeypatch.setattr(adjoint2d, "_record_monitors", lambda *a: [])
+    fake.timed_out = {late}
+    St = collections.namedtuple("St", adjoint2d.STATE_TM)
+    st = St(*[torch.zeros(6, 8)] * len(St._fields))
+    # 256-step chunks walked in pieces of 64, the first chunk from the imported state
+    monkeypatch.setattr(adjoint2d, "_cuts", lambda c, te: ((0, 0), (0, 0)))
+    g = adjoint2d.GradRun2D(st, types.SimpleNamespace(dt=0.1), 300, None, [], chunk=256)
+    g.eng, g.out_state, g.accs, g.snaps = _engine(fake, "fwd"), st, [], [[], []]
+    if late is None:
+        g.backward([None] * len(g.names))
+        assert plans == ["rec0", "rec1", "rec2"]
+        return
+    with pytest.raises(MtbError, match="bounded wait"):
+        g.backward([None] * len(g.names))
