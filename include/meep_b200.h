@@ -294,13 +294,18 @@ typedef struct mtb_tuning {
                                while per-launch timing is off), -1 off      */
     int32_t variant;        /* 2D: 0 default (where every structure is
                                eligible for 3: tiles resident for a ring of
-                               steps if each gets an SM of its own, else the
-                               cluster kernel or 3; otherwise 2), 1 row march, 2 one-step
-                               tiles, 3 temporally blocked tiles (up to 4
-                               steps per launch from TMA-staged 32 x 128
-                               tiles; PEC structures without conductivity,
-                               poles or magnetic pairs; the plan's first
-                               step runs on the one-step tiles);
+                               steps if each gets an SM of its own, else 4
+                               for TM plans of at most one cluster per 16
+                               SMs that fit it, else 3; otherwise 2),
+                               1 row march, 2 one-step tiles, 3 temporally
+                               blocked tiles (up to 4 steps per launch from
+                               TMA-staged 32 x 128 tiles; PEC structures
+                               without conductivity, poles or magnetic
+                               pairs; the plan's first step runs on the
+                               one-step tiles), 4 cluster kernel (TM
+                               structures eligible for 3, each in the shared
+                               memory of one cluster for a ring of steps;
+                               refused where one does not fit);
                                3D: 0 default (3 where it applies, from 8 M
                                cells and rows filled to 4/5; else 2),
                                1 fused x-march (register-staged), 2 split

@@ -2470,15 +2470,15 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
     if (n < 1 || !structs_in) return fail(MTB_INVALID_ARG, "need at least one structure");
     if (n_amp_cols < 0) return fail(MTB_INVALID_ARG, "n_amp_cols < 0");
     // default (0): after the first step, when every structure is eligible, the resident
-    // kernel where the tiles fit the GPU, else the temporally blocked kernels; 3: the
-    // temporally blocked ones; 4: small TM grids only (resident or the cluster kernel); 2: the
-    // one-step tiles only
+    // kernel where the tiles fit the GPU, else the cluster kernel for small TM plans, else the
+    // temporally blocked kernels; 3: the temporally blocked ones; 4: the cluster kernel,
+    // refused where a structure does not fit; 2: the one-step tiles only
     const int tv = tuning ? tuning->variant : 0;
     if (tv < 0 || tv > 4) return fail(MTB_INVALID_ARG, "2D variant %d not in 0..4", tv);
     const int variant = tv == 1 ? 1 : 2;
     bool want_tb = tv == 3 || tv == 0;
     bool want_cl = tv == 4 || tv == 0;
-    bool want_res = tv == 4 || tv == 0;
+    bool want_res = tv == 0;
     int rows = (tuning && tuning->rows_per_warp > 0) ? tuning->rows_per_warp : 32;
     int wr = 1;
     if (variant == 2) {
