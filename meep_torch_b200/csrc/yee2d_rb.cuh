@@ -81,19 +81,18 @@ struct RbTile {
 };
 
 // Where a thread's tile lies and what is valid there; rows are bit r + 1 of the masks
-// (bit 0: row -1, bit RW + 1: row RW). Validity is folded into coefficients, as in the
-// one-step tiles, so the update carries no predicates: a difference along y is scaled by
-// 1 / dx or, in a column that is not updated, 0; a row that is not updated has dt 0. Rows
-// and columns off the arrays hold zeros with 1/eps = 0 and stay zero.
+// (bit 0: row -1, bit RW + 1: row RW). A difference is set to +0 in a row or column that
+// is not updated (an and with its bits: a factor of 0 would give NaN beside a field that has
+// overflowed). Rows and columns off the arrays hold zeros with 1/eps = 0 and stay zero.
 template <int RW>
 struct RbPos {
     int nx, ny, P;
     int iw;                  // structure row of this warp's row 0
     int jb;                  // structure column of this lane's first cell
     int w, lane, W;
-    float ca[4], cb[4];      // masked 1 / dx per column: TM Hx, Dz; TE Dx, Hz
-    float ty[RW + 1];        // masked dt per row: TM Hy of rows -1 .. RW-1; TE Dy of 0 .. RW
-    float tm[RW];            // TM Dz; TE Hz
+    unsigned ca[4], cb[4];   // ~0 where the column is updated, else 0: TM Hx, Dz; TE Dx, Hz
+    unsigned ty[RW + 1];     // the same of rows: TM Hy of rows -1 .. RW-1; TE Dy of 0 .. RW
+    unsigned tm[RW];         // TM Dz; TE Hz
     unsigned rout;           // rows of the output block inside the grid (bit r)
     bool outc;               // columns of the output block inside the array
     bool act;                // columns inside the array
@@ -150,18 +149,18 @@ __device__ __forceinline__ RbPos<RW> rb_pos(const RbMeta &M, const int4 a, int r
     for (int q = 0; q < 4; ++q) {
         const int j = p.jb + q;
         const bool h = j >= 0 && j <= ny - 2, in = j >= 1 && j <= ny - 2;
-        p.ca[q] = (TE ? in : h) ? p.rdx : 0.f;
-        p.cb[q] = (TE ? h : in) ? p.rdx : 0.f;
+        p.ca[q] = (TE ? in : h) ? ~0u : 0u;
+        p.cb[q] = (TE ? h : in) ? ~0u : 0u;
     }
 #pragma unroll
     for (int r = 0; r <= RW; ++r) {
         const int i = p.iw + r - (TE ? 0 : 1);
-        p.ty[r] = (TE ? (i >= 1 && i <= nx - 2) : (i >= 0 && i <= nx - 2)) ? p.dt : 0.f;
+        p.ty[r] = (TE ? (i >= 1 && i <= nx - 2) : (i >= 0 && i <= nx - 2)) ? ~0u : 0u;
     }
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
         const int i = p.iw + r;
-        p.tm[r] = (TE ? (i >= 0 && i <= nx - 2) : (i >= 1 && i <= nx - 2)) ? p.dt : 0.f;
+        p.tm[r] = (TE ? (i >= 0 && i <= nx - 2) : (i >= 1 && i <= nx - 2)) ? ~0u : 0u;
     }
     p.rout = (rb_rows_in<RW>(p.iw, a.y, min(a.y + rows_out, nx) - 1) >> 1) & ((1u << RW) - 1);
     p.xb = 0;
@@ -234,7 +233,8 @@ __device__ __forceinline__ void rb_source(int which, const RbPos<RW> &p, const R
     float wv[4];
     lds4(sh.ws + which * sh.plane + row * RB_C + 4 * p.lane, wv);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = __fsub_rn(v[q], __fmul_rn(a, wv[q]));
+    for (int q = 0; q < 4; ++q)              // (an infinite amplitude leaves other cells alone)
+        v[q] = wv[q] != 0.f ? __fsub_rn(v[q], __fmul_rn(a, wv[q])) : v[q];
 }
 
 template <int RW>
@@ -301,6 +301,9 @@ __device__ __forceinline__ void rb_exchange(const RbShared &sh, const RbPos<RW> 
 __device__ __forceinline__ float rb_d(float a, float b, float rdx) {       // (a - b) / dx
     return __fmul_rn(__fsub_rn(a, b), rdx);
 }
+__device__ __forceinline__ float rb_and(float v, unsigned mask) {
+    return __uint_as_float(__float_as_uint(v) & mask);
+}
 // CPML term: t = d + q with q = b psi + a d (kappa = 1), psi <- q
 __device__ __forceinline__ float rb_cpml(float d, float b, float a, float &psi) {
     psi = __fmaf_rn(b, psi, __fmul_rn(a, d));
@@ -341,7 +344,8 @@ __device__ __forceinline__ void rb_step(RbTile<false, RW> &T, const RbMeta &M,
                                                      r < 0 ? T.iah[q] : T.ia[r < 0 ? 0 : r][q],
                                                      e1), rdx)
                                : rb_d(e1, e0, rdx);
-            h[q] = __fmaf_rn(p.ty[r + 1], XL ? rb_cpml(d, b, a, ps[q]) : d, h[q]);
+            const float t = rb_and(d, p.ty[r + 1]);
+            h[q] = __fmaf_rn(dt, XL ? rb_cpml(t, b, a, ps[q]) : t, h[q]);
         }
         if (XL) {
             if (r < 0) copy4(T.ph, ps);
@@ -361,11 +365,12 @@ __device__ __forceinline__ void rb_step(RbTile<false, RW> &T, const RbMeta &M,
             const float er = q < 3 ? T.e[r][q < 3 ? q + 1 : 3] : er4;
             constexpr int q1[4] = {1, 2, 3, 3};
             const float d =
-                !CL ? rb_d(er, T.e[r][q], p.ca[q])
+                !CL ? rb_d(er, T.e[r][q], rdx)
                 : (q == 0 || q == 3)
-                    ? __fmul_rn(__fmaf_rn(-T.m[r][q], T.ia[r][q], er), p.ca[q])
-                    : __fmul_rn(__fmaf_rn(T.m[r][q1[q]], T.ia[r][q1[q]], -T.e[r][q]), p.ca[q]);
-            T.x[r][q] = __fmaf_rn(-dt, YL ? rb_cpml(d, yb[q], ya[q], ps[q]) : d, T.x[r][q]);
+                    ? __fmul_rn(__fmaf_rn(-T.m[r][q], T.ia[r][q], er), rdx)
+                    : __fmul_rn(__fmaf_rn(T.m[r][q1[q]], T.ia[r][q1[q]], -T.e[r][q]), rdx);
+            const float c = rb_and(d, p.ca[q]);
+            T.x[r][q] = __fmaf_rn(-dt, YL ? rb_cpml(c, yb[q], ya[q], ps[q]) : c, T.x[r][q]);
         }
         if (YL) st4(psi + r * RB_C, ps);
     }
@@ -392,14 +397,16 @@ __device__ __forceinline__ void rb_step(RbTile<false, RW> &T, const RbMeta &M,
         for (int q = 0; q < 4; ++q) {
             const float ha = r > 0 ? T.y[r > 0 ? r - 1 : 0][q] : T.yh[q];
             const float hm = q > 0 ? T.x[r][q > 0 ? q - 1 : 0] : hm4;
-            const float dhy = rb_d(T.y[r][q], ha, p.cb[q]);
-            const float dhx = rb_d(T.x[r][q], hm, p.cb[q]);
+            const unsigned v = p.cb[q] & p.tm[r];
+            const float fy = rb_and(__fsub_rn(T.y[r][q], ha), v);
+            const float dhy = __fmul_rn(fy, rdx);
+            const float dhx = rb_and(rb_d(T.x[r][q], hm, rdx), v);
             const float ty = XL ? rb_cpml(dhy, b, a, p2[q]) : dhy;
             const float tx = YL ? rb_cpml(dhx, yb[q], ya[q], p3[q]) : dhx;
             const float c0 = __fsub_rn(ty, tx);
-            const float c1 = __fmaf_rn(__fsub_rn(T.y[r][q], ha), p.cb[q], -tx);
+            const float c1 = __fmaf_rn(fy, rdx, -tx);
             const float curl = (CL || YL) ? c0 : !XL ? c1 : ((p.xb >> r) & 1u) ? c0 : c1;
-            T.m[r][q] = __fmaf_rn(p.tm[r], curl, T.m[r][q]);
+            T.m[r][q] = __fmaf_rn(dt, curl, T.m[r][q]);
         }
         if (XL) st4(psi + 2 * sh.plane + r * RB_C, p2);
         if (YL) st4(psi + 3 * sh.plane + r * RB_C, p3);
@@ -443,8 +450,8 @@ __device__ __forceinline__ void rb_step(RbTile<true, RW> &T, const RbMeta &M,
         for (int q = 0; q < 4; ++q) {
             const float h1 = r == RW ? hb[q] : T.m[r < RW ? r : 0][q];
             const float h0 = r == 0 ? ha[q] : T.m[r > 0 ? r - 1 : 0][q];
-            const float d = rb_d(h1, h0, rdx);
-            h[q] = __fmaf_rn(-p.ty[r], XL ? rb_cpml(d, b, a, ps[q]) : d, h[q]);
+            const float d = rb_and(rb_d(h1, h0, rdx), p.ty[r]);
+            h[q] = __fmaf_rn(-dt, XL ? rb_cpml(d, b, a, ps[q]) : d, h[q]);
         }
         if (XL) {
             if (r == RW) copy4(T.ph, ps);
@@ -462,7 +469,7 @@ __device__ __forceinline__ void rb_step(RbTile<true, RW> &T, const RbMeta &M,
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const float hm = q > 0 ? T.m[r][q > 0 ? q - 1 : 0] : hm4;
-            const float d = rb_d(T.m[r][q], hm, p.ca[q]);
+            const float d = rb_and(rb_d(T.m[r][q], hm, rdx), p.ca[q]);
             T.x[r][q] = __fmaf_rn(dt, YL ? rb_cpml(d, yb[q], ya[q], ps[q]) : d, T.x[r][q]);
             ex[r][q] = __fmul_rn(T.x[r][q], T.ia[r][q]);
         }
@@ -496,19 +503,20 @@ __device__ __forceinline__ void rb_step(RbTile<true, RW> &T, const RbMeta &M,
             const float en = r + 1 < RW ? ey[r + 1 < RW ? r + 1 : 0][q] : eyb[q];
             const float exn = q < 3 ? ex[r][q < 3 ? q + 1 : 3] : ex4;
             constexpr int q1[4] = {1, 2, 3, 3};
+            const unsigned v = p.cb[q] & p.tm[r];
             const float fy = LEAN ? __fmaf_rn(-T.y[r][q], T.ib[r][q], en)
-                                  : __fsub_rn(en, ey[r][q]);
-            const float fx = !LEAN    ? __fsub_rn(exn, ex[r][q])
+                                  : rb_and(__fsub_rn(en, ey[r][q]), v);
+            const float fx = !LEAN    ? rb_and(__fsub_rn(exn, ex[r][q]), v)
                              : q == 3 ? __fmaf_rn(-T.x[r][q], T.ia[r][q], exn)
                                       : __fmaf_rn(T.x[r][q1[q]], T.ia[r][q1[q]], -ex[r][q]);
-            const float dey = __fmul_rn(fy, p.cb[q]);
-            const float dex = __fmul_rn(fx, p.cb[q]);
+            const float dey = __fmul_rn(fy, rdx);
+            const float dex = __fmul_rn(fx, rdx);
             const float ty = XL ? rb_cpml(dey, b, a, p2[q]) : dey;
             const float tx = YL ? rb_cpml(dex, yb[q], ya[q], p3[q]) : dex;
             const float c0 = __fsub_rn(ty, tx);
-            const float c1 = __fmaf_rn(fy, p.cb[q], -tx);
+            const float c1 = __fmaf_rn(fy, rdx, -tx);
             const float curl = YL ? c0 : !XL ? c1 : ((p.xb >> r) & 1u) ? c0 : c1;
-            T.m[r][q] = __fmaf_rn(-p.tm[r], curl, T.m[r][q]);
+            T.m[r][q] = __fmaf_rn(-dt, curl, T.m[r][q]);
         }
         if (XL) st4(psi + 2 * sh.plane + r * RB_C, p2);
         if (YL) st4(psi + 3 * sh.plane + r * RB_C, p3);

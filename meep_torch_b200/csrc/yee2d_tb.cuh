@@ -23,7 +23,7 @@
 //
 // What bounds it: instruction issue, 2-3 us per tile for taking, set-up and
 // storing and 1.0-1.4 us per sub-step (TM lean; 480 x 480). Per launch of 4
-// steps: 10 TM structures of about 512 x 512 78 -> 69 us, TE 90 -> 78 us, 64 TM
+// steps: 10 TM structures of about 512 x 512 78 -> 69 us, TE 90 -> 76 us, 64 TM
 // of 256 x 256 156 -> 153 us (all its tiles reach a y layer). The barriers
 // themselves cost little; registers do: 64 a thread, and each form below that
 // spilled more lost more than it saved.
@@ -695,17 +695,17 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
             }
             continue;
         }
-        // validity as factors: columns in 1 / dx (Dx; Hz), rows in dt (Dy; Hz). Where a factor is
-        // zero the operands are too (walls, padding) or the row is not used. (In k_tb_tm this
-        // form spilled: 167 against 155 us per launch of 64 structures of 256 x 256.)
+        // validity: a difference is 0 in a column that is not updated (Dx; Hz), and a row that
+        // is not updated is skipped, a branch of the whole warp (Dy; Hz). A factor of 0 in its
+        // place would give NaN on walls beside a field that has overflowed. The off-array
+        // operands of the other cells are zeros.
         unsigned mX = 0, mZ = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int j = jb + q;
             if (j >= 1 && j <= ny - 2) mX |= 1u << q;
-            if (j >= 0 && j <= ny - 2) mZ |= 1u << q;
+            if (hzRow && j >= 0 && j <= ny - 2) mZ |= 1u << q;
         }
-        const float ty = dyRow ? dt : 0.f, tz = hzRow ? dt : 0.f;
         const bool bxH = hzRow && in_band(i, S.xband[0], S.xband[1]);
         const bool bxE = dyRow && in_band(i, S.xband[2], S.xband[3]);
         const float *xpr = L.xprof + (k & 1) * 4 * TB_R + w;
@@ -732,8 +732,8 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                 if (YL) { lds4(yp0, p); lds4(pr + 2 * TB_C, b); lds4(pr + 3 * TB_C, a); }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    const float d = tb_d(hz[q], q > 0 ? hz[q > 0 ? q - 1 : 0] : hzL,
-                                         ((mX >> q) & 1u) ? rdx : 0.f);
+                    const float t = tb_d(hz[q], q > 0 ? hz[q > 0 ? q - 1 : 0] : hzL, rdx);
+                    const float d = ((mX >> q) & 1u) ? t : 0.f;
                     dx[q] = __fmaf_rn(dt, YL ? tb_cpml(d, b[q], a[q], p[q]) : d, dx[q]);
                     ex[q] = __fmul_rn(dx[q], ix[q]);
                 }
@@ -742,11 +742,13 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                 if (bxE) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
-                        dy[q] = __fmaf_rn(-ty, tb_cpml(tb_d(hz[q], ha[q], rdx), exb, exa, p1[q]), dy[q]);
+                        dy[q] = __fmaf_rn(-dt, tb_cpml(tb_d(hz[q], ha[q], rdx), exb, exa, p1[q]), dy[q]);
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        dy[q] = __fmaf_rn(-ty, tb_d(hz[q], ha[q], rdx), dy[q]);
+                    for (int q = 0; q < 4; ++q) {
+                        const float dn = __fmaf_rn(-dt, tb_d(hz[q], ha[q], rdx), dy[q]);
+                        dy[q] = dyRow ? dn : dy[q];
+                    }
                 }
                 if (srcE) apply_cells_rn(S.src_e, i, C.amp_e + s * C.ncols, jb, dy);
 #pragma unroll
@@ -762,19 +764,21 @@ __global__ void __launch_bounds__(TB_THREADS, 1) k_tb_te(
                 if (YL || bxH) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const float cz = ((mZ >> q) & 1u) ? rdx : 0.f;
-                        const float dey = tb_d(eb[q], ey[q], cz);
-                        const float dex = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], cz);
+                        const bool v = (mZ >> q) & 1u;
+                        const float ty = tb_d(eb[q], ey[q], rdx), dey = v ? ty : 0.f;
+                        const float tx = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], rdx);
+                        const float dex = v ? tx : 0.f;
                         const float t = bxH ? tb_cpml(dey, hxb, hxa, p2[q]) : dey;
                         const float u = YL ? tb_cpml(dex, b[q], a[q], p[q]) : dex;
-                        hz[q] = __fmaf_rn(-tz, __fsub_rn(t, u), hz[q]);
+                        hz[q] = __fmaf_rn(-dt, __fsub_rn(t, u), hz[q]);
                     }
                 } else {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const float cz = ((mZ >> q) & 1u) ? rdx : 0.f;
-                        const float dex = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], cz);
-                        hz[q] = __fmaf_rn(-tz, __fmaf_rn(__fsub_rn(eb[q], ey[q]), cz, -dex), hz[q]);
+                        const float dex = tb_d(q < 3 ? ex[q < 3 ? q + 1 : 3] : exR, ex[q], rdx);
+                        const float c = __fmaf_rn(__fsub_rn(eb[q], ey[q]), rdx, -dex);
+                        const float hn = __fmaf_rn(-dt, c, hz[q]);
+                        hz[q] = ((mZ >> q) & 1u) ? hn : hz[q];
                     }
                 }
                 if (YL) st4(yp3, p);
