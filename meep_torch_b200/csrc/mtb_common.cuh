@@ -85,18 +85,22 @@ struct StreamMarks {
     };
     std::vector<One> uses;
     bool unknown = false;            // captured by a caller, or an event failed: cannot tell
+    // a call that fails here fails for no caller: its error is not left for the next check
+    static bool did(cudaError_t e) noexcept {
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess;
+    }
     void mark(cudaStream_t st) noexcept {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (unknown) return;
         unknown = true;
-        if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
-            return;
+        if (!did(cudaStreamIsCapturing(st, &cs)) || cs != cudaStreamCaptureStatusNone) return;
         cudaEvent_t ev = nullptr;
         for (const One &u : uses)
             if (u.st == st) ev = u.ev;
         if (!ev) {
             if (uses.size() >= 16) return;
-            if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return;
+            if (!did(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming))) return;
             try {
                 uses.push_back({st, ev});
             } catch (...) {
@@ -104,13 +108,13 @@ struct StreamMarks {
                 return;
             }
         }
-        unknown = cudaEventRecord(ev, st) != cudaSuccess;
+        unknown = !did(cudaEventRecord(ev, st));
     }
     // waits for all of it; false if that cannot be told
     bool wait() noexcept {
         for (const One &u : uses) {
-            if (!unknown && cudaEventSynchronize(u.ev) != cudaSuccess) unknown = true;
-            cudaEventDestroy(u.ev);
+            if (!unknown && !did(cudaEventSynchronize(u.ev))) unknown = true;
+            did(cudaEventDestroy(u.ev));
         }
         uses.clear();
         return !unknown;
