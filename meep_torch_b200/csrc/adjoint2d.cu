@@ -802,6 +802,7 @@ int mtb_yee2d_adjoint_create(const mtb_yee2d_struct *s, const mtb_adj2d_buffers 
                                                                 ring_slot_elems, 4) * p->dft.slots);
         if (rc2) { p->dft.release(); delete p; return rc2; }
     }
+    p->marks.ready();
     *out = p;
     return MTB_OK;
 }

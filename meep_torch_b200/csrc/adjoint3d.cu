@@ -540,6 +540,7 @@ int mtb_yee3d_adjoint_create(const mtb_yee3d_struct *s, const mtb_adj3d_buffers 
         p->dft.release(); delete p;
         return fail(MTB_CUDA_ERROR, "3D adjoint upload: %s", cudaGetErrorString(e));
     }
+    p->marks.ready();
     *out = p;
     return MTB_OK;
 }

@@ -45,8 +45,8 @@ int profile_band(const float *b_d, const float *a_d, int n, int32_t &lo_end, int
 // Plan scratch comes from a bounded pool, so that building and closing a plan does not pay
 // cudaMalloc / cudaFree (and their pinned forms) a dozen times: these took 1.3 of the 3.3 ms of
 // a 200-step run of a small plan, and up to 10 ms where other programs use the driver too.
-// A block goes back only when the work of every stream its plan ran on has finished
-// (StreamMarks, ScratchIdle; not by a device-wide wait, which breaks graph captures of other
+// A block goes back only when its plan's set-up and the work of every stream it ran on have
+// finished (StreamMarks, ScratchIdle; not by a device-wide wait, which breaks graph captures of other
 // threads), so any thread, stream or plan of that device may take it next; contents are not
 // kept or cleared. Without that knowledge it is freed, as cudaFree waits by itself. At most
 // SCRATCH_KEEP bytes stay (the oldest blocks are freed first), none are kept when an
@@ -84,12 +84,16 @@ struct StreamMarks {
         cudaEvent_t ev;
     };
     std::vector<One> uses;
-    bool unknown = false;            // captured by a caller, or an event failed: cannot tell
+    // cannot tell: set-up not finished, captured by a caller, or a call failed
+    bool unknown = true;
     // a call that fails here fails for no caller: its error is not left for the next check
     static bool did(cudaError_t e) noexcept {
         if (e != cudaSuccess) cudaGetLastError();
         return e == cudaSuccess;
     }
+    // The end of the plan's creation: its copies (of pageable memory, on the legacy stream) may
+    // land after the calls that made them have returned. Before it, nothing is known to be idle.
+    void ready() noexcept { unknown = !did(cudaStreamSynchronize(cudaStreamLegacy)); }
     void mark(cudaStream_t st) noexcept {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (unknown) return;

@@ -2798,6 +2798,7 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
         mtb_yee2d_plan_destroy(p);
         return rc;
     }
+    p->marks.ready();
     *out = p;
     return MTB_OK;
 }

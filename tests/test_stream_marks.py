@@ -73,13 +73,19 @@ static bool idle(Work *w) { return w->done == w->queued; }
 int main(int, char **argv) {
     const char *what = argv[1];
     mtb::StreamMarks m;
-#ifdef MARKS_READY
+    if (!strcmp(what, "unfinished")) {           // set-up copies may still be landing
+        printf("%d\n", (int)!m.wait());
+        return 0;
+    }
+    work_of(cudaStreamLegacy)->queued += 2;      // set-up copies
     m.ready();
-#endif
-    bool ok = false;
+    bool ok = idle(work_of(cudaStreamLegacy));
+    if (!ok) return 1;
     if (!strcmp(what, "use")) {                  // work on two streams is waited for
         for (int k = 0; k < 2; ++k) { work_of(stream(k))->queued += 3; m.mark(stream(k)); }
         ok = m.wait() && idle(work_of(stream(0))) && idle(work_of(stream(1)));
+    } else if (!strcmp(what, "unused")) {        // set up, never run
+        ok = m.wait();
     } else if (!strcmp(what, "capture")) {       // captured work cannot be waited for
         work_of(stream(0))->capturing = true;
         m.mark(stream(0));
@@ -106,6 +112,6 @@ def marks(tmp_path_factory):
                                        check=True, timeout=60).stdout.strip()
 
 
-@pytest.mark.parametrize("what", ["use", "capture", "last_error"])
+@pytest.mark.parametrize("what", ["use", "capture", "last_error", "unfinished", "unused"])
 def test_marks(marks, what):
     assert marks(what) == "1"
