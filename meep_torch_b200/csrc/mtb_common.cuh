@@ -77,10 +77,11 @@ struct ScratchBuf {
 using DevBuf = ScratchBuf<false>;
 using HostBuf = ScratchBuf<true>;
 
-// The streams a plan has queued work on, each with an event behind its latest use.
+// The streams a plan has queued work on, each with an event behind its latest use. A stream
+// is known by its id: its handle may name another one after it is destroyed, work pending.
 struct StreamMarks {
     struct One {
-        cudaStream_t st;
+        unsigned long long id;
         cudaEvent_t ev;
     };
     std::vector<One> uses;
@@ -96,17 +97,19 @@ struct StreamMarks {
     void ready() noexcept { unknown = !did(cudaStreamSynchronize(cudaStreamLegacy)); }
     void mark(cudaStream_t st) noexcept {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
         if (unknown) return;
         unknown = true;
         if (!did(cudaStreamIsCapturing(st, &cs)) || cs != cudaStreamCaptureStatusNone) return;
+        if (!did(cudaStreamGetId(st, &id))) return;
         cudaEvent_t ev = nullptr;
         for (const One &u : uses)
-            if (u.st == st) ev = u.ev;
+            if (u.id == id) ev = u.ev;
         if (!ev) {
             if (uses.size() >= 16) return;
             if (!did(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming))) return;
             try {
-                uses.push_back({st, ev});
+                uses.push_back({id, ev});
             } catch (...) {
                 cudaEventDestroy(ev);
                 return;

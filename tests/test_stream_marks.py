@@ -84,6 +84,14 @@ int main(int, char **argv) {
     if (!strcmp(what, "use")) {                  // work on two streams is waited for
         for (int k = 0; k < 2; ++k) { work_of(stream(k))->queued += 3; m.mark(stream(k)); }
         ok = m.wait() && idle(work_of(stream(0))) && idle(work_of(stream(1)));
+    } else if (!strcmp(what, "reused")) {        // a stream destroyed, its handle used again
+        Work *gone = work_of(stream(0));
+        gone->queued = 5;
+        m.mark(stream(0));
+        handles.erase(stream(0));
+        work_of(stream(0))->queued = 2;
+        m.mark(stream(0));
+        ok = m.wait() && idle(gone) && idle(work_of(stream(0)));
     } else if (!strcmp(what, "unused")) {        // set up, never run
         ok = m.wait();
     } else if (!strcmp(what, "capture")) {       // captured work cannot be waited for
@@ -112,6 +120,7 @@ def marks(tmp_path_factory):
                                        check=True, timeout=60).stdout.strip()
 
 
-@pytest.mark.parametrize("what", ["use", "capture", "last_error", "unfinished", "unused"])
+@pytest.mark.parametrize("what", ["use", "capture", "last_error", "unfinished", "unused",
+                                  "reused"])
 def test_marks(marks, what):
     assert marks(what) == "1"
