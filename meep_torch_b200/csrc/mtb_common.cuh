@@ -87,6 +87,8 @@ struct StreamMarks {
     std::vector<One> uses;
     // cannot tell: set-up not finished, captured by a caller, or a call failed
     bool unknown = true;
+    bool open = false;               // work on open_st whose mark is still to come
+    cudaStream_t open_st = nullptr;
     // a call that fails here fails for no caller: its error is not left for the next check
     static bool did(cudaError_t e) noexcept {
         if (e != cudaSuccess) cudaGetLastError();
@@ -98,6 +100,8 @@ struct StreamMarks {
     void mark(cudaStream_t st) noexcept {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         unsigned long long id = 0;
+        if (open && open_st != st) unknown = true;
+        open = false;
         if (unknown) return;
         unknown = true;
         if (!did(cudaStreamIsCapturing(st, &cs)) || cs != cudaStreamCaptureStatusNone) return;
@@ -117,8 +121,20 @@ struct StreamMarks {
         }
         unknown = !did(cudaEventRecord(ev, st));
     }
+    // A use that the mark at the end of its chunk of steps will cover: an event for every half
+    // step would be one per launch. A chunk left unfinished cannot be told, nor one that
+    // changes streams (the first may be gone by then).
+    void later(cudaStream_t st) noexcept {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (open && open_st != st) unknown = true;
+        if (!did(cudaStreamIsCapturing(st, &cs)) || cs != cudaStreamCaptureStatusNone)
+            unknown = true;
+        open = true;
+        open_st = st;
+    }
     // waits for all of it; false if that cannot be told
     bool wait() noexcept {
+        unknown = unknown || open;
         for (const One &u : uses) {
             if (!unknown && !did(cudaEventSynchronize(u.ev))) unknown = true;
             did(cudaEventDestroy(u.ev));
@@ -133,6 +149,17 @@ struct MarkUse {
     cudaStream_t st;
     MarkUse(StreamMarks &marks, void *stream) : m(marks), st((cudaStream_t)stream) {}
     ~MarkUse() { m.mark(st); }
+};
+// the same for an entry point that makes one part of a chunk: marked when no part is left
+template <class Plan>
+struct MarkChunk {
+    Plan &p;
+    cudaStream_t st;
+    MarkChunk(Plan &plan, void *stream) : p(plan), st((cudaStream_t)stream) {}
+    ~MarkChunk() {
+        if (p.c_s < p.c_k) p.marks.later(st);
+        else p.marks.mark(st);
+    }
 };
 // while it lives, buffers that this thread releases are known to be idle (if `idle`)
 struct ScratchIdle {

@@ -1533,7 +1533,7 @@ int mtb_yee3d_set_slab(mtb_yee3d_plan *p, int32_t own_lo, int32_t own_hi) {
 
 int mtb_yee3d_begin(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
-    const MarkUse use(p->marks, stream);
+    const MarkChunk<mtb_yee3d_plan> use(*p, stream);
     if (int rc = need_split(p, "half steps")) return rc;
     if (k <= 0) return fail(MTB_INVALID_ARG, "k must be > 0");
     p->last_launches = 0;
@@ -1542,7 +1542,7 @@ int mtb_yee3d_begin(mtb_yee3d_plan *p, int64_t t0, int32_t k, const double *coef
 
 int mtb_yee3d_half(mtb_yee3d_plan *p, int32_t part, void *stream) {
     if (!p) return fail(MTB_INVALID_ARG, "plan is null");
-    const MarkUse use(p->marks, stream);
+    const MarkChunk<mtb_yee3d_plan> use(*p, stream);
     if (p->c_s >= p->c_k) return fail(MTB_INVALID_ARG, "no staged step left (mtb_yee3d_begin)");
     if (part != p->c_half)
         return fail(MTB_INVALID_ARG, "half %d out of order (expected %d)", part, p->c_half);

@@ -92,6 +92,26 @@ int main(int, char **argv) {
         work_of(stream(0))->queued = 2;
         m.mark(stream(0));
         ok = m.wait() && idle(gone) && idle(work_of(stream(0)));
+    } else if (!strcmp(what, "halves")) {        // one record for a chunk of half steps
+        for (int k = 0; k < 63; ++k) { ++work_of(stream(0))->queued; m.later(stream(0)); }
+        ++work_of(stream(0))->queued;
+        m.mark(stream(0));
+        ok = records == 1 && m.wait() && idle(work_of(stream(0)));
+    } else if (!strcmp(what, "halves_streams")) {   // a stream that may be gone by now
+        m.later(stream(0));
+        handles.clear();
+        m.mark(stream(1));
+        ok = handles.count(stream(0)) == 0 && !m.wait();
+    } else if (!strcmp(what, "halves_left")) {   // a chunk that was not finished
+        ++work_of(stream(0))->queued;
+        m.later(stream(0));
+        ok = !m.wait();
+    } else if (!strcmp(what, "halves_capture")) {
+        work_of(stream(0))->capturing = true;
+        m.later(stream(0));
+        work_of(stream(0))->capturing = false;
+        m.mark(stream(0));
+        ok = !m.wait();
     } else if (!strcmp(what, "unused")) {        // set up, never run
         ok = m.wait();
     } else if (!strcmp(what, "capture")) {       // captured work cannot be waited for
@@ -121,6 +141,7 @@ def marks(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what", ["use", "capture", "last_error", "unfinished", "unused",
-                                  "reused"])
+                                  "reused", "halves", "halves_streams", "halves_left",
+                                  "halves_capture"])
 def test_marks(marks, what):
     assert marks(what) == "1"
