@@ -172,8 +172,9 @@ struct ScratchIdle {
 // started (pdl_next) and SM space is free, and waits in pdl_wait until it has finished and
 // its writes are visible. So the launch latency and everything before pdl_wait overlap the
 // previous kernel. Rules: every thread that goes on calls pdl_wait before it reads or writes
-// what an earlier kernel of the chain wrote or reads; such data is not read through the
-// read-only path (__ldg, const __restrict__), which the wait does not order. Behind anything
+// what an earlier kernel of the chain wrote or reads, and at least one thread of every launch
+// does (so that a kernel's end implies that of all before it); such data is not read through
+// the read-only path (__ldg, const __restrict__), which the wait does not order. Behind anything
 // but a kernel (a copy, an event) the launch is an ordinary one. Measured, whole runs:
 // 400 x 301 TM with poles, 800 steps (one tile launch each, about 8 us) 11.4 -> 9.2 ms;
 // 117 x 90 x 75, 240 steps of three launches 11.7 -> 9.8 ms; 128 x 112 x 100 with poles

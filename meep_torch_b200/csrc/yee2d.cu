@@ -1049,9 +1049,9 @@ __device__ __forceinline__ void tm_tile(const mtb_yee2d_struct &S, const int i, 
     const float dt = S.dt, rdx = 1.0f / S.dx;
     const int par = C.par;
     const uint32_t ro = (uint32_t)i * P + jb;        // box < 2^31 cells (plan check)
-    const float *__restrict__ Dz = S.f_main[par];
-    const float *__restrict__ Hx = S.f_x[par];
-    const float *__restrict__ Hy = S.f_y[par];
+    const float *Dz = S.f_main[par];
+    const float *Hx = S.f_x[par];
+    const float *Hy = S.f_y[par];
     const float *__restrict__ ie = S.inv_eps_a;
     // symmetry cuts: the cut row (x) / column (y) of Dz is live
     const bool cutx = EXT && S.cut_x != 0, cuty = EXT && S.cut_y != 0;
@@ -1399,9 +1399,9 @@ __device__ __forceinline__ void te_tile(const mtb_yee2d_struct &S, const int i, 
     const float dt = S.dt, rdx = 1.0f / S.dx;
     const int par = C.par;
     const uint32_t ro = (uint32_t)i * P + jb;
-    const float *__restrict__ Hz = S.f_main[par];
-    const float *__restrict__ Dx = S.f_x[par];
-    const float *__restrict__ Dy = S.f_y[par];
+    const float *Hz = S.f_main[par];
+    const float *Dx = S.f_x[par];
+    const float *Dy = S.f_y[par];
     const float *__restrict__ iex = S.inv_eps_a;
     const float *__restrict__ iey = S.inv_eps_b;
     // even symmetry cuts (core/stepper_te.py:88-97): the cut row of Dy (x cut) and
@@ -1620,9 +1620,9 @@ __device__ __forceinline__ void tm_rows(const mtb_yee2d_struct &S, const int ib,
     const bool act = jb < P;
     const float dt = S.dt, rdx = 1.0f / S.dx;
     const int par = C.par;
-    const float *__restrict__ Dz = S.f_main[par];
-    const float *__restrict__ Hx = S.f_x[par];
-    const float *__restrict__ Hy = S.f_y[par];
+    const float *Dz = S.f_main[par];
+    const float *Hx = S.f_x[par];
+    const float *Hy = S.f_y[par];
     const float *__restrict__ ie = S.inv_eps_a;
     // lanes past the row end (last strip) read the row's last float4 instead:
     // their results are never stored and feed only masked neighbour cells
@@ -1852,9 +1852,9 @@ __device__ __forceinline__ void te_rows(const mtb_yee2d_struct &S, const int ib,
     const bool act = jb < P;
     const float dt = S.dt, rdx = 1.0f / S.dx;
     const int par = C.par;
-    const float *__restrict__ Hz = S.f_main[par];
-    const float *__restrict__ Dx = S.f_x[par];
-    const float *__restrict__ Dy = S.f_y[par];
+    const float *Hz = S.f_main[par];
+    const float *Dx = S.f_x[par];
+    const float *Dy = S.f_y[par];
     const float *__restrict__ iex = S.inv_eps_a;
     const float *__restrict__ iey = S.inv_eps_b;
     // lanes past the row end (last strip) read the row's last float4 instead:

@@ -675,8 +675,8 @@ __device__ __forceinline__ void s3_e(const Split3 &P, const S3Cell &c,
     constexpr int AB = C == 0 ? 2 : C == 1 ? 0 : 1;
     const bool pa_on = C == 0 ? (xok && by) : C == 1 ? (vyH && bz) : bx;
     const bool pb_on = C == 0 ? (xok && bz) : C == 1 ? (vyH && bx) : by;
-    const float *__restrict__ Ha = P.ho[FA];
-    const float *__restrict__ Hb = P.ho[FB];
+    const float *Ha = P.ho[FA];
+    const float *Hb = P.ho[FB];
     float ha[4], hap[4], hb[4], hbp[4], ep[4], epn[4], en[4], pa[4], pb[4];
     z4(ha); z4(hap); z4(hb); z4(hbp); one4(ep); one4(epn); z4(en); z4(pa); z4(pb);
     float zk = 0.f, epk = 1.f;                            // H(k-1) of q = 0, eps(k+1) of q = 3
