@@ -1,0 +1,1 @@
+from ._lib import release_scratch  # noqa: F401

@@ -238,6 +238,12 @@ def zero(lib, bufs, stream: int):
                        (C.c_int64 * n)(*[t.numel() for t in bufs]), n, stream), "mtb_zero")
 
 
+def release_scratch():
+    """Free the memory that closed plans left in the scratch pool (at most 256 MB of device
+    memory, which torch's allocator neither sees nor can take back, and 16 MB pinned)."""
+    load().mtb_release_scratch()
+
+
 def ptr(t) -> int:
     """Raw device pointer of a torch tensor (0 for None)."""
     return 0 if t is None else int(t.data_ptr())
