@@ -384,6 +384,11 @@ int mtb_yee2d_run_noalloc(const mtb_yee2d_struct *s, const mtb_dft_region *regio
  * spin forever; a wait that gives up sets this flag and the step returns. */
 int mtb_yee2d_check(mtb_yee2d_plan *plan, void *stream);
 
+/* Device address of that flag (0, or not 0 after an expired wait), valid while the plan
+ * lives: for programs that read it in stream order instead of waiting. Accumulators and
+ * gathered samples are NaN once it is raised, in 2D and 3D plans. */
+int mtb_yee2d_error_flag(const mtb_yee2d_plan *plan, const int32_t **flag);
+
 /* Number of kernel launches the last mtb_yee2d_run issued. */
 int64_t mtb_yee2d_last_launches(const mtb_yee2d_plan *plan);
 

@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(CT, 3) k_dft_contract(
     const mtb_dft_region *__restrict__ regions, const int *__restrict__ blk_region,
     const int64_t *__restrict__ blk_start, const int *__restrict__ group_nf,
     const int *__restrict__ group_off, int total_nf, const float *__restrict__ phase, int row0,
-    int n, const float *__restrict__ ring, int64_t slot_elems, int64_t n_chunks) {
+    int n, const float *__restrict__ ring, int64_t slot_elems, int64_t n_chunks,
+    const int *__restrict__ err) {
     extern __shared__ float4 sP4[];
     float2 *sP = reinterpret_cast<float2 *>(sP4);
     const int64_t per = (n_chunks + gridDim.x - 1) / gridDim.x;
@@ -344,10 +345,12 @@ __global__ void __launch_bounds__(CT, 3) k_dft_contract(
             if (staged != 2 * R.group + (sel >> 1)) {
                 staged = 2 * R.group + (sel >> 1);
                 const float *p0 = phase + ((int64_t)row0 * total_nf + group_off[R.group]) * 4 + sel;
+                // after an expired wait the samples are incomplete: NaN phases, so NaN sums
+                const bool bad = err && *err;
                 for (int e = threadIdx.x; e < n * (fb - fa); e += CT) {
                     const int s = e / (fb - fa), f = e - s * (fb - fa);
                     const float *p = p0 + ((int64_t)s * total_nf + fa + f) * 4;
-                    sP[f * (n + 2) + s] = make_float2(p[0], p[1]);
+                    sP[f * (n + 2) + s] = bad ? make_float2(NAN, NAN) : make_float2(p[0], p[1]);
                 }
                 __syncthreads();
             }
@@ -700,8 +703,7 @@ int DftState::contract(int row0, int n, cudaStream_t st, LaunchTimer *tm,
     k_dft_contract<<<dim3((unsigned)nb, fsplit), CT, smem, st>>>(
         regions_d.as<mtb_dft_region>(), blk_region_d.as<int>(), blk_start_d.as<int64_t>(), gd,
         gd + (n_groups + 1), total_nf, phase_base ? phase_base : phase_d.as<float>(), row0, n,
-        ring_d.as<float>(),
-        slot_elems, n_blocks);
+        ring_d.as<float>(), slot_elems, n_blocks, wait_err);
     MTB_CHECK_LAUNCH();
     if (tm && (rc = tm->end(st))) return rc;
     return MTB_OK;

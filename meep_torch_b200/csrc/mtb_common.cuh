@@ -270,6 +270,7 @@ struct DftState {
     // device
     DevBuf regions_d, blk_start_d, blk_region_d, phase_d, ring_d;
     DevBuf freq_dt_d;                      // {frequency, dt} of every phase column
+    const int *wait_err = nullptr;         // the plan's flag of expired waits, if it has one
     PinnedPair phase_h;
     int64_t slot_elems = 0;
     int slots = 0;                         // ring depth K

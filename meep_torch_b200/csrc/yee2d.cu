@@ -2798,8 +2798,15 @@ int mtb_yee2d_plan_create(const mtb_yee2d_struct *structs_in, int32_t n,
         mtb_yee2d_plan_destroy(p);
         return rc;
     }
+    p->dft.wait_err = p->err_d.as<int>();
     p->marks.ready();
     *out = p;
+    return MTB_OK;
+}
+
+int mtb_yee2d_error_flag(const mtb_yee2d_plan *p, const int32_t **flag) {
+    if (!p || !flag) return fail(MTB_INVALID_ARG, "error flag: null plan or output");
+    *flag = p->err_d.as<int32_t>();
     return MTB_OK;
 }
 
@@ -2890,15 +2897,16 @@ static int launch_step(mtb_yee2d_plan *p, const Ctx2D &C, cudaStream_t st) {
     return MTB_OK;
 }
 
-// out[s * n_off + j] = ring slot s at offset off[j]; offsets outside the slot read 0.
+// out[s * n_off + j] = ring slot s at offset off[j]; offsets outside the slot read 0. NaN
+// after an expired wait (the samples are incomplete).
 __global__ void k_ring_gather(const float *__restrict__ ring, int64_t slot_elems,
                               const int64_t *__restrict__ off, int n_off, int n_slots,
-                              float *__restrict__ out) {
+                              float *__restrict__ out, const int *__restrict__ err) {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= (int64_t)n_off * n_slots) return;
     const int s = (int)(e / n_off), j = (int)(e - (int64_t)s * n_off);
     const int64_t o = off[j];
-    out[e] = (o >= 0 && o < slot_elems) ? ring[s * slot_elems + o] : 0.f;
+    out[e] = *err ? NAN : (o >= 0 && o < slot_elems) ? ring[s * slot_elems + o] : 0.f;
 }
 
 // One TB launch pair (TM tiles, then TE tiles) advancing C.nsub steps.
@@ -3516,7 +3524,8 @@ int mtb_yee2d_ring_gather(const mtb_yee2d_plan *p, const int64_t *offsets, int32
     const int64_t n = (int64_t)n_off * n_slots;
     const MarkUse use(p->marks, stream);
     k_ring_gather<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        p->dft.ring_d.as<float>(), p->dft.slot_elems, offsets, n_off, n_slots, out);
+        p->dft.ring_d.as<float>(), p->dft.slot_elems, offsets, n_off, n_slots, out,
+        p->err_d.as<int>());
     MTB_CHECK_LAUNCH();
     return MTB_OK;
 }
@@ -3574,7 +3583,7 @@ __global__ void k_dft_contract(const mtb_dft_region *__restrict__ regions,
                                const int *__restrict__ group_nf, const int *__restrict__ group_off,
                                int total_nf, const float *__restrict__ phase, int row0, int n,
                                const float *__restrict__ ring, int64_t slot_elems,
-                               int64_t n_chunks);
+                               int64_t n_chunks, const int *__restrict__ err);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[MTB_NOALLOC_SCRATCH_BYTES];
 constexpr int NA_MAX_DEV = 64;
@@ -3970,7 +3979,7 @@ extern "C" int mtb_yee2d_run_noalloc(const mtb_yee2d_struct *s, const mtb_dft_re
                 k_dft_contract<<<(unsigned)std::min<int64_t>(n_blocks, 148 * 16), NA_CT,
                                  sizeof(float2) * (slot + 2) * maxnf, st>>>(
                     dReg, dBlk, dBs, dGnf, dGoff, total_nf, dPhase, q + 1 - slot, slot, dRing,
-                    ring_slot_elems, n_blocks);
+                    ring_slot_elems, n_blocks, nullptr);
                 MTB_CHECK_LAUNCH();
                 slot = 0;
             } else if (slot == ring_slots || q == n - 1) {

@@ -1375,6 +1375,7 @@ int mtb_yee3d_plan_create(const mtb_yee3d_struct *s, const mtb_dft_region *regio
         mtb_yee3d_plan_destroy(p);
         return fail(MTB_CUDA_ERROR, "plan upload failed: %s", cudaGetErrorString(e));
     }
+    p->dft.wait_err = p->err_d.as<int>();         // (null without the one-pass kernel)
     p->marks.ready();
     *out = p;
     return MTB_OK;

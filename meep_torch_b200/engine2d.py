@@ -1009,13 +1009,18 @@ class Engine2D:
             psi_Hxy=self._unpack(ps[3][cur], (nx_e, ny_e), (xoff, yoff)))
 
     def accumulators(self, b: int = 0):
-        """Structure b's accumulators, one per monitor (the plan's own buffers). Checks the
-        run first (see check()), unless the plan's stream is being captured."""
-        with torch.cuda.stream(self.stream):
-            capturing = torch.cuda.is_current_stream_capturing()
-        if not capturing:
+        """Structure b's accumulators, one per monitor (the plan's own buffers, still being
+        formed while the run is on its stream). After an expired wait they are NaN, and a run
+        that has finished is checked here (see check()); a pending one is not waited for."""
+        if not getattr(self, "_checked", False) and self._finished():
             self.check()
         return list(self.items[b].accs)
+
+    def _finished(self) -> bool:
+        """The plan's stream has run all of its work (False under capture)."""
+        with torch.cuda.stream(self.stream):
+            return not torch.cuda.is_current_stream_capturing() and \
+                torch.cuda.current_stream(self.device).query()
 
     def close(self):
         if getattr(self, "plan", None):

@@ -88,12 +88,9 @@ class _Lib:
 
 @pytest.fixture
 def fake(monkeypatch):
-    import torch
-
     from meep_torch_b200 import _lib as L
     lib = _Lib()
     monkeypatch.setattr(L, "load", lambda: lib)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     return lib
 
 
@@ -121,16 +118,15 @@ def _engine(lib, plan, nx=6, ny=8):
     return e
 
 
-def test_accumulators_report_a_timeout(fake, monkeypatch):
-    import torch
-
+def test_accumulators_report_a_timeout(fake):
     from meep_torch_b200._lib import MtbError
     fake.timed_out = {"p"}
     e = _engine(fake, "p")
+    e._finished = lambda: True
     with pytest.raises(MtbError, match="bounded wait"):
         e.accumulators(0)
-    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
-    assert len(e.accumulators(0)) == 1               # no synchronisation in a capture
+    e._finished = lambda: False
+    assert len(e.accumulators(0)) == 1       # pending or captured: not waited for (NaN then)
     e.plan = None
 
 
@@ -164,3 +160,43 @@ def test_gradient_reports_a_timeout_of_any_recording_plan(fake, monkeypatch, lat
         return
     with pytest.raises(MtbError, match="bounded wait"):
         g.backward([None] * len(g.names))
+
+
+# ------------------------------------------------------------------ what the flag does
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", [0, 2, 3, 4])
+@pytest.mark.parametrize("ring", [32, 7])
+def test_raised_flag_turns_accumulators_into_nan(variant, ring):
+    """The flag is raised by the test (no wait is made to expire): the sums of the run that
+    follows are NaN and the run is reported."""
+    import ctypes as C
+
+    import torch
+
+    from meep_torch_b200 import _lib as L
+    from meep_torch_b200.core.coeffs import build_tm_coeffs
+    from meep_torch_b200.core.grid import Grid
+    from meep_torch_b200.core.monitors import DFTFieldsMonitor, FluxMonitorTM
+    from meep_torch_b200.core.sources import GaussianPulse, LineSource
+    from meep_torch_b200.core.stepper_tm import init_tm_state
+    from meep_torch_b200.engine2d import Engine2D
+    nx, ny = 70, 60
+    g = Grid(nx=nx, ny=ny, dx=0.05, device="cuda")
+    m = build_tm_coeffs(g, eps_inf=torch.full((nx, ny), 2.0, device="cuda"), npml=8)
+    src = LineSource(g, ix=20, j0=10, j1=50, profile=GaussianPulse(0.6, 0.4))
+    mons = [DFTFieldsMonitor(g, [0.5, 0.6, 0.7, 0.8, 0.9], "Ez"),
+            FluxMonitorTM(g, [0.5], x_normal=True, idx=40, lo=10, hi=50)]
+    e = Engine2D([(init_tm_state(g), m, src, mons)], variant=variant, ring_slots=ring)
+    e.run(0, 40)
+    torch.cuda.synchronize()
+    assert all(torch.isfinite(a).all() for a in e.accumulators(0))
+    flag, one = C.c_void_p(), torch.ones(1, device="cuda")
+    L.check(e.lib.mtb_yee2d_error_flag(e.plan, C.byref(flag)))
+    L.check(e.lib.mtb_pack(L.ptr(one), 1, 1, 1, 1, 1, flag, 1, 1, 1, 1, 1, 0, 0, 0, e._sptr()))
+    e.run(40, 40)
+    accs = list(e.items[0].accs)
+    torch.cuda.synchronize()
+    assert all(torch.isnan(a).all() for a in accs)
+    with pytest.raises(L.MtbError):
+        e.accumulators(0)
+    e.close()
