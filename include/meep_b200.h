@@ -384,6 +384,10 @@ int mtb_yee2d_run_noalloc(const mtb_yee2d_struct *s, const mtb_dft_region *regio
  * spin forever; a wait that gives up sets this flag and the step returns. */
 int mtb_yee2d_check(mtb_yee2d_plan *plan, void *stream);
 
+/* The same without waiting: *finished is 0 where work on `stream` is pending (or captured),
+ * and nothing is reported; else 1, and as mtb_yee2d_check. */
+int mtb_yee2d_poll(mtb_yee2d_plan *plan, void *stream, int32_t *finished);
+
 /* Device address of that flag (0, or not 0 after an expired wait), valid while the plan
  * lives: for programs that read it in stream order instead of waiting. Accumulators and
  * gathered samples are NaN once it is raised, in 2D and 3D plans. */

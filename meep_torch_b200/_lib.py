@@ -136,6 +136,7 @@ SIGNATURES = {
     "mtb_yee2d_set_timing": (C.c_int, [vp, C.c_int32]),
     "mtb_yee2d_timing": (C.c_int, [vp, C.POINTER(C.c_double), C.POINTER(C.c_int64),
                                    C.POINTER(C.c_double), C.POINTER(C.c_int64)]),
+    "mtb_yee2d_poll": (C.c_int, [vp, vp, C.POINTER(C.c_int32)]),
     "mtb_yee2d_error_flag": (C.c_int, [vp, C.POINTER(vp)]),
     "mtb_yee3d_plan_create": (C.c_int, [C.POINTER(Yee3DStruct), C.POINTER(DftRegion), C.c_int32,
                                         C.POINTER(PhaseGroup), C.c_int32, C.c_int64,

@@ -77,6 +77,15 @@ struct ScratchBuf {
 using DevBuf = ScratchBuf<false>;
 using HostBuf = ScratchBuf<true>;
 
+// While it lives, this thread's synchronising calls are allowed beside graph captures of other
+// threads (in the default capture mode these forbid them to every thread, and end broken).
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    BesideCaptures(const BesideCaptures &) = delete;
+};
+
 // The streams a plan has queued work on, each with an event behind its latest use. A stream
 // is known by its id: its handle may name another one after it is destroyed, work pending.
 struct StreamMarks {

@@ -2822,6 +2822,19 @@ int mtb_yee2d_check(mtb_yee2d_plan *p, void *stream) {
     return MTB_OK;
 }
 
+int mtb_yee2d_poll(mtb_yee2d_plan *p, void *stream, int32_t *finished) {
+    if (!p || !finished) return fail(MTB_INVALID_ARG, "poll: null plan or output");
+    const BesideCaptures beside;
+    const cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    *finished = 0;
+    if (!StreamMarks::did(cudaStreamIsCapturing(st, &cs)) || cs != cudaStreamCaptureStatusNone)
+        return MTB_OK;
+    if (!StreamMarks::did(cudaStreamQuery(st))) return MTB_OK;      // pending
+    *finished = 1;
+    return mtb_yee2d_check(p, stream);
+}
+
 // One step's kernels on `st`.
 static int launch_step(mtb_yee2d_plan *p, const Ctx2D &C, cudaStream_t st) {
     const int n_tm = p->n_work_tm, n_te = p->n_work - p->n_work_tm;

@@ -1012,15 +1012,12 @@ class Engine2D:
         """Structure b's accumulators, one per monitor (the plan's own buffers, still being
         formed while the run is on its stream). After an expired wait they are NaN, and a run
         that has finished is checked here (see check()); a pending one is not waited for."""
-        if not getattr(self, "_checked", False) and self._finished():
-            self.check()
+        if not getattr(self, "_checked", False):
+            done = C.c_int32()
+            L.check(self.lib.mtb_yee2d_poll(self.plan, self._sptr(), C.byref(done)),
+                    "mtb_yee2d_poll")
+            self._checked = bool(done.value)
         return list(self.items[b].accs)
-
-    def _finished(self) -> bool:
-        """The plan's stream has run all of its work (False under capture)."""
-        with torch.cuda.stream(self.stream):
-            return not torch.cuda.is_current_stream_capturing() and \
-                torch.cuda.current_stream(self.device).query()
 
     def close(self):
         if getattr(self, "plan", None):

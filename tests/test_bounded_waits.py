@@ -75,9 +75,14 @@ class _Lib:
 
     def __init__(self, timed_out=()):
         self.timed_out = set(timed_out)
+        self.pending = False
 
     def mtb_yee2d_check(self, plan, stream):
         return 3 if plan in self.timed_out else 0
+
+    def mtb_yee2d_poll(self, plan, stream, finished):
+        finished._obj.value = not self.pending
+        return 0 if self.pending else self.mtb_yee2d_check(plan, stream)
 
     def mtb_last_error(self):
         return b"a bounded wait expired"
@@ -122,11 +127,12 @@ def test_accumulators_report_a_timeout(fake):
     from meep_torch_b200._lib import MtbError
     fake.timed_out = {"p"}
     e = _engine(fake, "p")
-    e._finished = lambda: True
     with pytest.raises(MtbError, match="bounded wait"):
         e.accumulators(0)
-    e._finished = lambda: False
-    assert len(e.accumulators(0)) == 1       # pending or captured: not waited for (NaN then)
+    fake.pending = True                      # or captured: not waited for (NaN then)
+    assert len(e.accumulators(0)) == 1 and not e._checked
+    fake.pending, fake.timed_out = False, set()
+    assert len(e.accumulators(0)) == 1 and e._checked
     e.plan = None
 
 
