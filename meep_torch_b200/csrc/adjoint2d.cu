@@ -691,7 +691,9 @@ static int adjoint_chunk(mtb_yee2d_adjoint *p, int k, const float *rec, int64_t 
                 k_adj_tm_e<<<grid, blk, 0, st>>>(S, p->b, radj, rq + rec_offset[0], q & 1);
                 MTB_CHECK_LAUNCH();
             }
-            if ((rc = launch_pdl(S.n_mpoles > 0 ? k_adj_tm_h<true> : k_adj_tm_h<false>, grid, blk, st, S, p->b, radj))) return rc;
+            if ((rc = launch_pdl(S.n_mpoles > 0 ? k_adj_tm_h<true> : k_adj_tm_h<false>, grid, blk,
+                                 st, S, p->b, radj)))
+                return rc;
             if (q > 0)
                 rc = launch_pdl(k_adj_tm_eze, grid, blk, st, S, p->b, radj_of(q - 1),
                                 rec_of(q - 1) + rec_offset[0], (q - 1) & 1);
@@ -702,7 +704,8 @@ static int adjoint_chunk(mtb_yee2d_adjoint *p, int k, const float *rec, int64_t 
                 k_adj_te_h<<<grid, blk, 0, st>>>(S, p->b, radj);
                 MTB_CHECK_LAUNCH();
             }
-            if ((rc = launch_pdl(S.n_poles + S.n_poles_y > 0 ? k_adj_te_e<true> : k_adj_te_e<false>, grid, blk, st, S, p->b, radj, rq + rec_offset[0],
+            if ((rc = launch_pdl(S.n_poles + S.n_poles_y > 0 ? k_adj_te_e<true> : k_adj_te_e<false>,
+                                 grid, blk, st, S, p->b, radj, rq + rec_offset[0],
                                  rq + rec_offset[1])))
                 return rc;
             if (q > 0)

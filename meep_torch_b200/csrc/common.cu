@@ -301,15 +301,16 @@ constexpr int CT = 256;        // channels per contraction block
 // A chunk is CT channels of one region (the region of a chunk from a per-chunk table); a
 // block folds a contiguous range of chunks. Phase values of a region's (group, toff) are
 // staged in shared memory, frequency by frequency (sP[(f - fa) * (n + 2) + s] = (Re, Im);
-// the two spare columns spread the staging stores over the banks), and staged again only where the range enters a region of another group or time offset.
+// the two spare columns spread the staging stores over the banks), and staged again only
+// where the range enters a region of another group or time offset.
 //
 // What bounds it: memory, given enough loads in flight. A block per chunk spent its time in
 // the chain table -> region -> phases -> samples -> accumulators, one frequency after the
 // other (bends batch, 5.3 M channels: 285 us per 32-step flush, 3.2 TB/s). Now a block's
 // first chain serves all of its chunks, and the accumulators of NFC frequencies are loaded
 // with the samples, the next NFC before the last ones are stored; the region sits in shared
-// memory, since in registers it spilled. Now 214 us (4.2 TB/s; 64 designs: 203 ->
-// 151 us, 256^3 flux faces 59 -> 40 us, 24 frequencies of a flux line 6.8 -> 5.5 us).
+// memory, since in registers it spilled. Now 215 us (4.2 TB/s; 64 designs: 199 ->
+// 152 us, 256^3 flux faces 59 -> 40 us, 50 frequencies of a flux line 6.5 -> 5.5 us).
 constexpr int NFC = 4;
 constexpr int KFULL = 32;      // ring depth with a fully unrolled contraction (the default)
 constexpr int SB = 16;         // samples in flight at other depths

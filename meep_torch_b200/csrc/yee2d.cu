@@ -2184,20 +2184,15 @@ static int d2h_floats(std::vector<float> &h, const float *d, int n, int s) {
     return MTB_OK;
 }
 
-// Tensor maps, per-structure records (descriptor + line samples), padded
-// profiles and the tile list (TM tiles first, then TE) of a TB plan. A
-// structure's padded profiles are 4 y rows (hy b, a; ey b, a) of pitch + 128
-// floats, column j at index j + 4, then 4 x rows (hx b, a; ex b, a) of
-// nx + 32 floats, row i at index i + 4; inert (1, 0) off the arrays.
 // Orders n tiles (work items from `first`) so that the blocks' shares cost the same: block b
 // of a grid of g takes tiles b, b + g, b + 2g, ... In the order of rows and columns a share
 // is one column of tiles whenever g is a multiple of the tiles per row, and a tile that
 // reaches a y layer costs 1.8 (TM) to 2.1 (TE) times a lean one: the last of 148 blocks ended
 // after 65 us where the mean ended after 44 us (12 structures of 480 x 480; with the balance a
-// launch takes 52 us in place of 66). Each wave of g
-// tiles keeps its tiles (neighbours share their halos through L2); within a wave the costliest
-// tile goes to the block with the least so far. The last, partial wave is the blocks' first g'
-// by construction, so it is counted first.
+// launch takes 52 us in place of 66). Each wave of g tiles keeps its tiles (neighbours share
+// their halos through L2); within a wave the costliest tile goes to the block with the least
+// so far. The last, partial wave is the blocks' first g' by construction, so it is counted
+// first.
 static void tb_balance(std::vector<int4> &work, int first, int n, int g) {
     struct Tile { int cost; int4 rec[TB_WORK]; };
     if (n <= g) return;
@@ -2231,6 +2226,11 @@ static void tb_balance(std::vector<int4> &work, int first, int n, int g) {
     for (int w0 = 0; w0 < full; w0 += g) wave(w0, g);
 }
 
+// Tensor maps, per-structure records (descriptor + line samples), padded
+// profiles and the tile list (TM tiles first, then TE) of a TB plan. A
+// structure's padded profiles are 4 y rows (hy b, a; ey b, a) of pitch + 128
+// floats, column j at index j + 4, then 4 x rows (hx b, a; ex b, a) of
+// nx + 32 floats, row i at index i + 4; inert (1, 0) off the arrays.
 static int tb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs) {
     const int n = (int)structs.size();
     std::vector<CUtensorMap> maps((size_t)n * TBM_N);
@@ -3152,9 +3152,12 @@ static int rb_flags(const mtb_yee2d_struct &S, const mtb_line_sample *ls, int r0
 // Resident kernel: records, tile list (TM first, then TE), neighbours and flags. Taken when
 // the tiles of each polarisation fit the GPU at once, one block per SM (24 x 120 output
 // cells a tile at most: about 426 k cells); leaves p->res false otherwise. The line lies
-// where a second tile per SM would begin: below it a step costs 1.5-2.7 us here against
-// 3.3-4.3 us with launches of four steps or the cluster kernel; past it the blocks could
-// not all be resident, which their waits on one another need.
+// where a second tile per SM would begin: below it a step costs 1.5-2.6 us here against
+// 3.3-4.2 us with launches of four steps or the cluster kernel; past it the blocks could
+// not all be resident, which their waits on one another need. The ring's depth, the most
+// steps a launch can take, is no condition: at 1 / 4 / 32 steps a whole step of 600 x 400 TM
+// takes 16.6 / 6.3 / 3.1 us here and 16.6 / 7.5 / 5.0 us in launches of up to four steps, of
+// 320 x 160 TM 14.5 / 5.3 / 2.6 against 22.8 / 10.3 / 5.5 us with the cluster kernel.
 static int rb_setup_plan(mtb_yee2d_plan *p, const std::vector<mtb_yee2d_struct> &structs,
                          const std::vector<mtb_line_sample> &lines) {
     const int n = (int)structs.size();
@@ -3365,9 +3368,8 @@ int mtb_yee2d_run(mtb_yee2d_plan *p, int64_t t0, int32_t k, const double *coef_e
     cudaStream_t st = (cudaStream_t)stream;
     int rc;
     // the row march's bounded waits may have raised the error flag (the TB and resident
-    // kernels' flag is read by mtb_yee2d_check, which the engine calls when it exports the
-    // state; the one-step
-    // tiles and the cluster kernel never wait)
+    // kernels' flag is read by the contraction, and by mtb_yee2d_check when the engine exports
+    // the state; the one-step tiles and the cluster kernel never wait)
     if (p->variant == 1 && (rc = mtb_yee2d_check(p, stream))) return rc;
     const int nc = std::max(p->n_cols, 1);
     const size_t per = (size_t)k * nc;

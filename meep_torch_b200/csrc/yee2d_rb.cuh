@@ -18,12 +18,14 @@
 //
 // What bounds it, and why this split: small plans are chains of short dependent steps.
 // Launches of one or four steps (5.8-16.6 us each) or two cluster barriers a step (3.3 us)
-// set their time, not bytes. Per step, profiler, before -> with this kernel: 200 x 120 TM
-// 3.3 -> 1.47 us (cluster kernel before), 320 x 160 TM 4.34 -> 2.03 us (cluster kernel),
-// 501 x 389 TE 4.15 -> 2.67 us (temporally blocked kernel). About 0.25 us of each step is
+// set their time, not bytes. Per step, profiler, before -> with this kernel: 64 x 48 TM
+// 3.28 -> 1.46 us (cluster kernel before), 320 x 160 TM 4.16 -> 2.14 us (cluster kernel),
+// 501 x 389 TE 4.11 -> 2.58 us (temporally blocked kernel). About 0.25 us of each step is
 // the exchange between blocks every RB_T steps, the rest the warps' dependent updates and
-// the one barrier. The rounding of every sub-step is that of the kernel it stands in for
-// (CL: the cluster kernel; else the temporally blocked tile around it): same bits.
+// the one barrier (issue slots 22-34 % active, the barrier the largest stall). The rounding
+// of every sub-step is that of the kernel it stands in for (CL: the cluster kernel; else the
+// temporally blocked tile around it): same bits, but for a source cell listed more than
+// once, which is subtracted once with the summed weight.
 //
 // CPML memory sits in shared memory, each thread's own slots (no exchange), and only in
 // tiles that reach a layer; tiles that reach no x / no y layer run sub-steps without the
@@ -289,8 +291,8 @@ __device__ __forceinline__ void rb_exchange(const RbShared &sh, const RbPos<RW> 
 }
 
 // The update's rounding is written out (no contraction is left to the compiler) and is that
-// of the kernel which runs the same plan launch by launch, so that results stay the same
-// bit for bit whichever advances it (a term with psi = 0 adds 0 exactly):
+// of the kernel which would run the same plan launch by launch, so that results are the same
+// bit for bit whichever of the two advances it (a term with psi = 0 adds 0 exactly):
 //  - the temporally blocked kernels: tiles here never straddle one of their 24 x 120 output
 //    blocks; where a row has no term of a layer (no y layer in the tile, the row outside the
 //    x layer) the curl is one fma, else a difference of the two rounded terms; their lean TE

@@ -265,7 +265,7 @@ __device__ __forceinline__ void tb_take_psi(const float *ps, int flags, int w, i
 }
 
 // (a - b) / dx; the CPML term d + q with q = b psi + a d (kappa = 1), psi <- q. Rounding is
-// spelled out here and in the sub-steps: all 2D kernels give a plan the same bits.
+// spelled out here and in the sub-steps, so that the resident kernel can round alike.
 __device__ __forceinline__ float tb_d(float a, float b, float rdx) {
     return __fmul_rn(__fsub_rn(a, b), rdx);
 }
