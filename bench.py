@@ -1332,8 +1332,11 @@ def main():
             traffic = entry.get("dram_bytes_per_launch")
     e2e_val = (total_updates / r["e2e_s"] / 1e9
                if r["e2e_s"] == r["e2e_s"] else None)
-    kernel = ("k_cl_tm (cluster-resident, a ring of steps per launch; graph replays, step "
-              "time = run time / steps)" if args.workload == "cfg1" and args.variant in (0, 4)
+    kernel = ("k_rb_resident (resident tiles, a ring of steps per launch; graph replays, step "
+              "time = run time / steps)" if args.workload == "cfg1" and args.variant == 0
+              else
+              "k_cl_tm (cluster-resident, a ring of steps per launch; graph replays, step "
+              "time = run time / steps)" if args.workload == "cfg1" and args.variant == 4
               else
               "k_tb_tm (temporally blocked, 4 steps per launch; graph replays, step time = "
               "run time / steps)" if args.workload == "cfg1" and args.variant == 3 else
