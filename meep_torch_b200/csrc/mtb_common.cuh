@@ -46,9 +46,9 @@ int profile_band(const float *b_d, const float *a_d, int n, int32_t &lo_end, int
 // cudaMalloc / cudaFree (and their pinned forms) a dozen times: these took 1.3 of the 3.3 ms of
 // a 200-step run of a small plan, and up to 10 ms where other programs use the driver too.
 // A block goes back only when its plan's set-up and the work of every stream it ran on have
-// finished (StreamMarks, ScratchIdle; not by a device-wide wait, which breaks graph captures of other
-// threads), so any thread, stream or plan of that device may take it next; contents are not
-// kept or cleared. Without that knowledge it is freed, as cudaFree waits by itself. At most
+// finished (StreamMarks, ScratchIdle; not by a device-wide wait, which breaks graph captures
+// of other threads), so any thread, stream or plan of that device may take it next; contents
+// are not kept or cleared. Without that knowledge it is freed, as cudaFree waits by itself. At most
 // SCRATCH_KEEP bytes stay (the oldest blocks are freed first), none are kept when an
 // allocation fails, and mtb_release_scratch() frees all.
 constexpr size_t SCRATCH_KEEP[2] = {(size_t)256 << 20, (size_t)16 << 20};   // device, pinned

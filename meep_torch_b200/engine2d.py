@@ -1012,7 +1012,7 @@ class Engine2D:
         """Structure b's accumulators, one per monitor (the plan's own buffers, still being
         formed while the run is on its stream). After an expired wait they are NaN, and a run
         that has finished is checked here (see check()); a pending one is not waited for."""
-        if not getattr(self, "_checked", False):
+        if self.plan and not getattr(self, "_checked", False):
             done = C.c_int32()
             L.check(self.lib.mtb_yee2d_poll(self.plan, self._sptr(), C.byref(done)),
                     "mtb_yee2d_poll")

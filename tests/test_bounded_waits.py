@@ -133,7 +133,9 @@ def test_accumulators_report_a_timeout(fake):
     assert len(e.accumulators(0)) == 1 and not e._checked
     fake.pending, fake.timed_out = False, set()
     assert len(e.accumulators(0)) == 1 and e._checked
-    e.plan = None
+    e._checked, fake.timed_out = False, {"p", None}
+    e.close()
+    assert len(e.accumulators(0)) == 1       # a closed plan's are still there
 
 
 @pytest.mark.parametrize("late", [None, "rec0", "rec1", "rec2"])
